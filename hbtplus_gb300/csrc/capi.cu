@@ -64,7 +64,7 @@ static void carve(Carver &cv, Ctx &c, Staging &sg, long long N, long long S, boo
   c.plan_inter = cv.take<long long>(S);
   c.small_next = cv.take<int>(1);
   c.part_info = cv.take<int>(8 * S);
-  c.chunk_bbox = cv.take<unsigned>(6 * maxchunks);
+  c.seg_bbox = cv.take<unsigned>(6 * S);
   c.chunk_sums = cv.take<double>(24 * maxchunks);
   c.sb.lo_a = cv.take<unsigned long long>(N);
   c.sb.lo_b = cv.take<unsigned long long>(N);

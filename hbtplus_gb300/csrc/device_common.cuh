@@ -129,6 +129,12 @@ __device__ __forceinline__ unsigned float_key(float e)
   unsigned u = __float_as_uint(e == 0.f ? 0.f : e);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+__device__ __forceinline__ float key_float(unsigned k)
+{
+  return __uint_as_float((k & 0x80000000u) ? k & 0x7fffffffu : ~k);
+}
+// A subhalo's bounding box before any particle: keys above / below every float's.
+constexpr unsigned kBoxLow = 0xffffffffu, kBoxHigh = 0u;
 
 __device__ __forceinline__ int upper_bound_i(const int *a, int n, int x)
 {
@@ -167,7 +173,7 @@ struct Ctx {
   int opt_leaf_runs;                         // warp schedule streams all-particle cells
   int opt_schedule;                          // FP32 walk: 0 one walk per lane, 1 warp schedule
   int *part_info;                            // 8 ints per segment
-  unsigned *chunk_bbox;                      // 6 per chunk
+  unsigned *seg_bbox;                        // 6 per segment: float_key of the box's low and high corners
   double *chunk_sums;                        // 16 per chunk
   // sort
   SortBuffers sb;

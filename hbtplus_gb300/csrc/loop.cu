@@ -177,6 +177,11 @@ __global__ void k_init(Ctx c, const float *pos, const float *vel, const float *m
   c.epos_of_pid[i] = i;
   SegState &sg = c.seg[s];
   if (id[i] == sg.mb_id) atomicMin(&sg.first_mb, i - sg.off);
+  if (i == sg.off)
+    for (int j = 0; j < 3; j++) {
+      c.seg_bbox[6 * (size_t)s + j] = kBoxLow;
+      c.seg_bbox[6 * (size_t)s + 3 + j] = kBoxHigh;
+    }
 }
 
 // ---------------------------------------------------------------- plans
@@ -532,6 +537,17 @@ __global__ void __launch_bounds__(kLB) k_avg_chunks(Ctx c)
 }
 
 // ---------------------------------------------------------------- control
+// Sum k of subhalo s's chunks, in chunk order: one serial chain of double adds
+// (the order fixes the rounding), about 145 cycles each whatever runs ahead of
+// it (loads 16 at a time: no faster).
+__device__ __forceinline__ double sum_chunks(const Ctx &c, int s, int k)
+{
+  double t = 0.;
+  for (int b = c.bchunk_base[s]; b < c.bchunk_base[s + 1]; b++)
+    t += c.chunk_sums[(size_t)b * kSums + k];
+  return t;
+}
+
 __global__ void k_control(Ctx c, int max_passes)
 {
   HBTU_KERNEL_PROLOGUE();
@@ -542,15 +558,11 @@ __global__ void k_control(Ctx c, int max_passes)
   SegState &sg = c.seg[s];
   if (sg.status != SEG_ACTIVE) return;
   const int nb = c.part_info[8 * s + 7];
-  double part = 0.;
-  if (nb > 1 && lane < 7)
-    for (int b = c.bchunk_base[s]; b < c.bchunk_base[s + 1]; b++)
-      part += c.chunk_sums[(size_t)b * kSums + lane];
-  double v[7];
-#pragma unroll
-  for (int k = 0; k < 7; k++) v[k] = __shfl_sync(0xffffffffu, part, k);
+  const double part = nb > 1 && lane < 7 ? sum_chunks(c, s, lane) : 0.;
+  double mean[6];
+  const double mass = frame_means(part, lane, nb, mean);
   if (lane != 0) return;
-  control_segment(c, sg, nb, v, max_passes);
+  control_segment(c, sg, nb, mass, mean, max_passes);
 }
 
 // ---------------------------------------------------------------- block sorts
@@ -721,13 +733,16 @@ __global__ void k_final_seg(Ctx c, hbtu_result *res)
   const SegState &sg = c.seg[s];
   const DevParams &P = c.P;
   const bool summed = sg.status != SEG_TRIVIAL && sg.status != SEG_DISRUPTED;
-  double part = 0.;
-  if (summed && lane < 18)
-    for (int b = c.bchunk_base[s]; b < c.bchunk_base[s + 1]; b++)
-      part += c.chunk_sums[(size_t)b * kSums + lane];
+  const double part = summed && lane < 18 ? sum_chunks(c, s, lane) : 0.;
   double v[18];
 #pragma unroll
   for (int k = 0; k < 18; k++) v[k] = __shfl_sync(0xffffffffu, part, k);
+  // the divisions by the mass, one per lane: E, 1/2 (for K), the angular momentum
+  const double num = lane == 0 ? v[0] : (lane == 1 ? 0.5 : (lane < 5 ? part : 1.));
+  const double quot = ddiv(num, summed && sg.nbound > 1 && lane < 5 ? v[5] : 1.);
+  double over_m[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) over_m[k] = __shfl_sync(0xffffffffu, quot, k);
   if (lane != 0) return;
   hbtu_result r;
   memset(&r, 0, sizeof(r));
@@ -781,12 +796,11 @@ __global__ void k_final_seg(Ctx c, hbtu_result *res)
       r.mostbound_vel[2] = u.z;
     }
     if (sg.nbound > 1) {
-      const double M = v[5];
-      const double E = ddiv(v[0], M);
-      const double K = dmul(v[1], ddiv(0.5, M));
+      const double E = over_m[0];
+      const double K = dmul(v[1], over_m[1]);
       r.specific_potential = __double2float_rn(dsub(E, K));
       r.specific_kinetic = __double2float_rn(K);
-      for (int j = 0; j < 3; j++) r.specific_angmom[j] = __double2float_rn(ddiv(v[2 + j], M));
+      for (int j = 0; j < 3; j++) r.specific_angmom[j] = __double2float_rn(over_m[2 + j]);
     }
     for (int t = 0; t < 6; t++) {
       r.nbound_type[t] = (int64_t)v[6 + t];
@@ -836,9 +850,7 @@ __global__ void k_segsum_combine(Ctx c, double *out)
   HBTU_KERNEL_PROLOGUE();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= c.S) return;
-  double t = 0.;
-  for (int b = c.bchunk_base[s]; b < c.bchunk_base[s + 1]; b++) t += c.chunk_sums[(size_t)b * kSums];
-  out[s] = t;
+  out[s] = sum_chunks(c, s, 0);
 }
 
 __device__ int get_all_chunks(const Ctx &c, int s, int *v)

@@ -128,11 +128,24 @@ __device__ __forceinline__ void frame_terms(float4 a, float4 u, float4 o, const 
   }
 }
 
+// The bound block's mass-weighted means of a frame, by one warp: lanes 0..6
+// hold its sums (mass, mass-weighted velocity, mass-weighted position about
+// Elist[0]; v * m and x * m over m), and each lane divides one of them, so that
+// the warp issues one double division, not six.  Returns the mass.
+__device__ __forceinline__ double frame_means(double sum, int lane, int nb, double (&mean)[6])
+{
+  const double mass = __shfl_sync(0xffffffffu, sum, 0);
+  const double q = ddiv(sum, nb > 1 && lane < 7 ? mass : 1.);
+#pragma unroll
+  for (int k = 0; k < 6; k++) mean[k] = __shfl_sync(0xffffffffu, q, k + 1);
+  return mass;
+}
+
 // The decisions of subhalo s after a pass whose partition kept nb particles
-// bound; v[0..6] are the bound block's sums (mass, mass-weighted velocity,
-// mass-weighted position about Elist[0]) when nb > 1.
-__device__ __forceinline__ void control_segment(const Ctx &c, SegState &sg, int nb,
-                                                const double (&v)[7], int max_passes)
+// bound; msum and mean are the bound block's mass and means (frame_means)
+// when nb > 1.
+__device__ __forceinline__ void control_segment(const Ctx &c, SegState &sg, int nb, double msum,
+                                                const double (&mean)[6], int max_passes)
 {
   const DevParams &P = c.P;
   const int nl = sg.nlast;
@@ -174,13 +187,12 @@ __device__ __forceinline__ void control_segment(const Ctx &c, SegState &sg, int 
     sg.ref_pos[1] = a.y;
     sg.ref_pos[2] = a.z;
   } else if (nb > 1) {
-    const double msum = v[0];
     sg.mbound = (float)msum;
-    for (int j = 0; j < 3; j++) sg.ref_vel[j] = __double2float_rn(ddiv(v[1 + j], msum));
+    for (int j = 0; j < 3; j++) sg.ref_vel[j] = __double2float_rn(mean[j]);
     const float4 o = c.pm[c.epid[sg.off]];
     const double org[3] = {o.x, o.y, o.z};
     for (int j = 0; j < 3; j++) {
-      double x = ddiv(v[4 + j], msum);
+      double x = mean[3 + j];
       if (P.periodic) x = dadd(x, org[j]);
       sg.ref_pos[j] = __double2float_rn(x);
     }

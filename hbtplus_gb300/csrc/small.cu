@@ -465,7 +465,15 @@ __global__ void __launch_bounds__(kSB) k_unbind_small(Ctx c, int cap, int max_pa
       const int nb = partition(c, sg, P0, reinterpret_cast<long long *>(key0), val0, val1);
       double v[7];
       frame_sums(c, sg, nb, chunk, v);
-      if (threadIdx.x == 0) control_segment(c, sg, nb, v, max_passes);
+      if (threadIdx.x < 32) {
+        double sum = 0.;
+#pragma unroll
+        for (int k = 0; k < 7; k++)
+          if ((int)threadIdx.x == k) sum = v[k];
+        double mean[6];
+        const double mass = frame_means(sum, threadIdx.x, nb, mean);
+        if (threadIdx.x == 0) control_segment(c, sg, nb, mass, mean, max_passes);
+      }
       __syncthreads();
     }
   }

@@ -84,11 +84,17 @@ __global__ void __launch_bounds__(kTB) k_bbox_chunks(Ctx c)
     const int j = threadIdx.x;
     float v = sh[j][0];
     for (int k = 1; k < kTB / 32; k++) v = j < 3 ? fminf(v, sh[j][k]) : fmaxf(v, sh[j][k]);
-    c.chunk_bbox[(size_t)b * 6 + j] = __float_as_uint(v);
+    // the extremes of a subhalo's chunks do not depend on their order
+    unsigned *box = c.seg_bbox + 6 * (size_t)s + j;
+    if (j < 3)
+      atomicMin(box, float_key(v));
+    else
+      atomicMax(box, float_key(v));
   }
 }
 
-// Root cube of each active subhalo (seg_cube) from its chunks' boxes.
+// Root cube of each active subhalo (seg_cube) from its box, which is cleared
+// for the next pass.
 __global__ void k_cube(Ctx c)
 {
   HBTU_KERNEL_PROLOGUE();
@@ -96,17 +102,16 @@ __global__ void k_cube(Ctx c)
   if (s >= c.S) return;
   SegState &sg = c.seg[s];
   if (sg.status != SEG_ACTIVE) return;
+  const bool empty = c.tchunk_base[s + 1] == c.tchunk_base[s];
+  unsigned *box = c.seg_bbox + 6 * (size_t)s;
   float mn[3], mx[3];
-  const int b0 = c.tchunk_base[s], b1 = c.tchunk_base[s + 1];
   for (int j = 0; j < 3; j++) {
-    mn[j] = INFINITY;
-    mx[j] = -INFINITY;
-    for (int b = b0; b < b1; b++) {
-      mn[j] = fminf(mn[j], __uint_as_float(c.chunk_bbox[(size_t)b * 6 + j]));
-      mx[j] = fmaxf(mx[j], __uint_as_float(c.chunk_bbox[(size_t)b * 6 + 3 + j]));
-    }
+    mn[j] = empty ? INFINITY : key_float(box[j]);
+    mx[j] = empty ? -INFINITY : key_float(box[3 + j]);
+    box[j] = kBoxLow;
+    box[3 + j] = kBoxHigh;
   }
-  const int levels = seg_cube(sg, mn, mx, b1 == b0, c.P);
+  const int levels = seg_cube(sg, mn, mx, empty, c.P);
   atomicMax(&c.plan->max_levels, levels);
 }
 

@@ -25,6 +25,30 @@ namespace hbtu {
 
 __device__ __forceinline__ int ll_tz(long long v) { return v ? __ffsll(v) - 1 : 64; }
 
+// A double in units of 2^-E, if an integer below 2^62 there (else false).
+__device__ __forceinline__ bool double_fixed(double d, int E, long long &X)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+  const int ex = (int)((b >> 52) & 0x7ffull);
+  unsigned long long v = b & 0xfffffffffffffull;
+  if (ex == 0) {  // zero (a subnormal is no multiple of any unit used here)
+    X = 0;
+    return v == 0ull;
+  }
+  if (ex == 0x7ff) return false;
+  v |= 1ull << 52;
+  const int sh = ex - 1075 + E;
+  if (sh >= 0) {
+    if (sh > 9) return false;
+    v <<= sh;
+  } else {
+    if (-sh > 52 || (v & ((1ull << -sh) - 1ull)) != 0ull) return false;
+    v >>= -sh;
+  }
+  X = (long long)(b >> 63 ? 0ull - v : v);
+  return true;
+}
+
 // Fixed-point form of the key computation.  The reference halves the cube in
 // double: centre_k = centre_{k-1} +- len / 2^(k+1).  When the centre, len/4
 // and every later increment are integers in units of 2^-E, and every centre
@@ -35,20 +59,16 @@ __device__ __forceinline__ void fixed_point_cube(SegState &sg, int levels)
 {
   sg.kfast = 0;
   if (levels <= 0 || !(sg.len > 0.)) return;
-  double M = sg.len;
-  for (int j = 0; j < 3; j++) M = fmax(M, fabs(sg.center[j]) + sg.len);
-  int top;
-  frexp(M, &top);                // M < 2^top
-  const int E = 61 - top;        // |values| < 2^61 in fixed point
-  const double l4 = ldexp(sg.len, E - 2);
-  const double lmin = ldexp(sg.len, E - levels - 1);
-  if (l4 != trunc(l4) || lmin != trunc(lmin) || l4 >= 0x1p62) return;
-  const long long inc = (long long)l4;
+  long long M = 0;  // largest |centre| + len, as the bits of a positive double
+  for (int j = 0; j < 3; j++)
+    M = max(M, __double_as_longlong(dadd(fabs(sg.center[j]), sg.len)));
+  const int top = (int)(M >> 52) - 1022;  // the largest is below 2^top
+  const int E = 61 - top;                 // |values| < 2^61 in fixed point
+  long long inc, least;
+  if (!double_fixed(sg.len, E - 2, inc) || !double_fixed(sg.len, E - levels - 1, least)) return;
   int g = ll_tz(inc >> (levels - 1));  // trailing zeros of the smallest increment
   for (int j = 0; j < 3; j++) {
-    const double cj = ldexp(sg.center[j], E);
-    if (cj != trunc(cj) || fabs(cj) >= 0x1p62) return;
-    sg.kc[j] = (long long)cj;
+    if (!double_fixed(sg.center[j], E, sg.kc[j])) return;
     g = min(g, ll_tz(sg.kc[j]));
   }
   if (top + E - g > 53) return;  // some centre would need more than 53 bits
@@ -81,33 +101,54 @@ __device__ __forceinline__ bool float_fixed(float x, int E, long long &X)
   return true;
 }
 
+// x / 2, on the exponent where that is exact.
+__device__ __forceinline__ double half_of(double x)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned ex = (unsigned)(b >> 52) & 0x7ffu;
+  if (ex - 2u < 0x7ffu - 2u) return __longlong_as_double((long long)(b - (1ull << 52)));
+  return dmul(0.5, x);
+}
+
+// Depth of geometric subdivision of a cube of side len: the number of
+// halvings until the side is below res (the len halving rule of
+// src/gravity_tree.cpp:37-40), at most kMaxLevels, from exponents and mantissas.
+__device__ __forceinline__ int cube_levels(double len, float res)
+{
+  const unsigned long long a = (unsigned long long)__double_as_longlong(len);
+  const unsigned long long r = (unsigned long long)__double_as_longlong(f2d(res));
+  const int ea = (int)(a >> 52), er = (int)(r >> 52);
+  if (ea > 0 && ea < 0x7ff && er > 0 && er < 0x7ff) {
+    const unsigned long long low = 0xfffffffffffffull;
+    return min(kMaxLevels, max(0, ea - er + ((a & low) >= (r & low) ? 1 : 0)));
+  }
+  int levels = 0;
+  while (len >= (double)res && levels < kMaxLevels) {
+    len = dmul(len, 0.5);
+    levels++;
+  }
+  return levels;
+}
+
 // Root cube of a subhalo from the float bounding box of its tree particles
 // (src/oct_tree.tpp:30-51; an empty box gives a cube of side 0) and its depth
-// of geometric subdivision: the first level whose side is below
-// TreeNodeResolution (the len halving rule of src/gravity_tree.cpp:37-40).
+// of geometric subdivision.  One thread does this per subhalo and pass, so the
+// few double operations left (the sums and differences) matter: the halvings,
+// comparisons and fixed-point forms are integer operations.
 // The frame centre of the relative coordinates is the subhalo's frame.
 __device__ __forceinline__ int seg_cube(SegState &sg, const float mn[3], const float mx[3],
                                         bool empty, const DevParams &P)
 {
-  double xmin[3], xmax[3];
+  double Len = 0.;
   for (int j = 0; j < 3; j++) {
-    xmin[j] = mn[j];
-    xmax[j] = mx[j];
+    const double lo = f2d(mn[j]), hi = f2d(mx[j]);
+    const double e = dsub(hi, lo);
+    if (j == 0 || __double_as_longlong(e) > __double_as_longlong(Len)) Len = e;  // e >= 0
+    sg.center[j] = half_of(dadd(hi, lo));
   }
-  double Len = dsub(xmax[0], xmin[0]);
-  for (int j = 1; j < 3; j++) {
-    const double e = dsub(xmax[j], xmin[j]);
-    if (e > Len) Len = e;
-  }
-  for (int j = 0; j < 3; j++) sg.center[j] = dmul(0.5, dadd(xmax[j], xmin[j]));
   if (empty) Len = 0.;
   sg.len = Len;
-  int levels = 0;
-  double L = Len;
-  while (L >= (double)P.res && levels < kMaxLevels) {
-    L = dmul(L, 0.5);
-    levels++;
-  }
+  const int levels = cube_levels(Len, P.res);
   sg.levels = levels;
   fixed_point_cube(sg, levels);
   for (int j = 0; j < 3; j++) sg.fc[j] = sg.ref_pos[j];
@@ -233,13 +274,28 @@ __device__ __forceinline__ void cells_elem(const Ctx &c, int base, int n, int e,
 // Walk record meta of a cell with side^2 = l2 (float, as the reference
 // computes len*len): the squared distances below which the cell surely opens
 // and above which it surely does not, l2/theta^2 (1 -+ 1e-5); in between the
-// walk takes the reference's decision in double.  Particles (never opened)
+// walk takes the reference's decision in double, so these need be no better
+// than a small part of 1e-5 and are formed in float.  Particles (never opened)
 // get -1 for both.
 __device__ __forceinline__ int4 cell_meta(float l2, int skip, const DevParams &P)
 {
-  const double q = (double)l2 / (double)P.theta2;
-  const float lo = (float)(q * (1.0 - 1e-5)), hi = (float)(q * (1.0 + 1e-5));
-  return make_int4(__float_as_int(l2), skip, __float_as_int(lo), __float_as_int(hi));
+  const float q = __fdiv_rn(l2, P.theta2);
+  return make_int4(__float_as_int(l2), skip, __float_as_int(q * (1.f - 1e-5f)),
+                   __float_as_int(q * (1.f + 1e-5f)));
+}
+
+// Side of a cell at octal depth od, as float: the root's side halved od times
+// in double.  Every cell's depth is at most the subhalo's depth of geometric
+// subdivision, so each halving applies; it is exact, and taken on the
+// exponent (double arithmetic runs at 1/64 of the FP32 rate on this GPU).
+__device__ __forceinline__ float cell_side(double len, int od)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(len);
+  const int ex = (int)(b >> 52);
+  if (ex - od > 1023 - 120 && ex < 0x7ff)
+    return d2f(__longlong_as_double((long long)(b - ((unsigned long long)od << 52))));
+  for (int k = 0; k < od; k++) len = dmul(len, 0.5);
+  return __double2float_rn(len);
 }
 
 __device__ __forceinline__ int4 particle_meta(int skip)
@@ -309,10 +365,7 @@ __device__ __forceinline__ void cellnodes_elem(const Ctx &c, const SegState &sg,
   const long long xb = Xs[0];
   const int idx = lo + (int)(Xs[lo] - xb) + rank;
   const int skip = hi + 1 + (int)(Xs[hi + 1] - xb);
-  double len = sg.len;
-  for (int k = 0; k < od; k++)
-    if (len >= (double)c.P.res) len = dmul(len, 0.5);
-  const float lf = (float)len;
+  const float lf = cell_side(sg.len, od);
   c.nd[nb + idx].m = cell_meta(fmul(lf, lf), hi + 1 < n ? nb + skip : kDone, c.P);
   c.cidx[e] = nb + idx;
   c.cskip[e] = nb + skip;
@@ -328,35 +381,58 @@ __device__ __forceinline__ void cellnodes_elem(const Ctx &c, const SegState &sg,
   }
 }
 
-// 1/m to within a few units in the last place: the hardware's approximate
-// double reciprocal refined by two Newton-Raphson steps r <- r + r (1 - m r)
-// (each step squares the relative error).  ok: the residual 1 - m r, taken
-// once more, shows a relative error below 2^-49 (else r is not used).
+// 1/m for the quotients below, m > 0: the float reciprocal approximation,
+// refined by one Newton-Raphson step r <- r + r (1 - m r) in double, which
+// squares its relative error (at most 2^-22.4, with the rounding of m to float)
+// to below 2^-44.  ok: m lies in the range where none of this can overflow or
+// lose bits to subnormals (else r is not used).
 __device__ __forceinline__ double recip_refined(double m, bool &ok)
 {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(m));
-  r = __fma_rn(r, __fma_rn(-m, r, 1.0), r);
-  r = __fma_rn(r, __fma_rn(-m, r, 1.0), r);
-  ok = fabs(__fma_rn(-m, r, 1.0)) < 0x1p-49;
-  return r;
+  const float mf = d2f(m);
+  const unsigned ex = __float_as_uint(mf) >> 23;  // the sign bit too: a negative m is not ok
+  ok = ex - (127u - 100u) <= 200u;
+  float r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(mf));
+  const double r = f2d(r0);
+  return __fma_rn(r, __fma_rn(-m, r, 1.0), r);
 }
 
 // float(c / m) with the quotient first rounded to double, as the reference
 // rounds its double centre of mass to float, given r ~ 1/m (ok as above).
-// q = c * r then lies within a few double units in the last place of the
-// correctly rounded quotient, so both round to the same float unless q lies
-// within 64 units of a point halfway between two floats (its low 29 mantissa
-// bits near 2^28), or outside the range of normal floats; those take the
-// exact division.
+// q = c * r is within 2^-44 of c / m, at most 512 of its units in the last
+// place, so both round to the same float unless q lies that close to a
+// point M halfway between two floats (its low 29 mantissa bits near 2^28).
+// There (always, for instance, at the midpoint of two equal masses) the side
+// of M follows from rho = c - M m, one fused multiply-add: its sign and a zero
+// are exact.  c / m = M: a tie, to even.  |rho| at least 4 times the half
+// unit of M times m: the double quotient lies on rho's side of M.  In between,
+// and outside the range of normal floats, the exact division.  A cell of two
+// equal masses takes 12 to 15 double operations in all, where the
+// division's own (per axis, for the whole warp when one lane needs it)
+// more than doubled that: double runs at 1/64 of the FP32 rate on this GPU.
 __device__ __forceinline__ float quot_float(double c, double m, double r, bool ok)
 {
   const double q = dmul(c, r);
   const unsigned long long b = (unsigned long long)__double_as_longlong(q);
   const int ex = (int)((b >> 52) & 0x7ffull);
   const unsigned rem = (unsigned)(b & 0x1fffffffull);
-  if (ok && ex >= 1023 - 125 && ex <= 1023 + 126 && rem - (0x10000000u - 64u) > 128u)
-    return d2f(q);
+  if (ok && ex >= 1023 - 125 && ex <= 1023 + 126) {
+    if (rem - (0x10000000u - 512u) > 1024u) return d2f(q);
+    const unsigned long long mid = (b & ~0x1fffffffull) | 0x10000000ull;
+    const unsigned long long rho = (unsigned long long)__double_as_longlong(
+        __fma_rn(-__longlong_as_double((long long)mid), m, c));
+    // 4 * (half a unit of M) * m, by its exponent: 2^(ex - 1023 - 53 + 2) m
+    const unsigned long long far = (unsigned long long)__double_as_longlong(m) +
+                                   ((unsigned long long)(long long)(ex - 1023 - 51) << 52);
+    const unsigned long long arho = rho & 0x7fffffffffffffffull;
+    if (arho == 0ull || arho >= far) {
+      const unsigned long long down = (mid & 0x7fffffffffffffffull) >> 29;  // towards zero
+      const bool up = arho == 0ull ? (down & 1ull) != 0ull : (rho >> 63) == (mid >> 63);
+      const unsigned bits =
+          (unsigned)(down - ((unsigned long long)(1023 - 127) << 23)) + (up ? 1u : 0u);
+      return __uint_as_float(bits | ((unsigned)(mid >> 63) << 31));
+    }
+  }
   return d2f(ddiv(c, m));
 }
 
