@@ -465,6 +465,14 @@ DevParams derive_params(const hbtu_params &p)
   d.maxsample = p.max_sample_size;
   d.h = 2.8 * (double)d.eps;
   d.h_inv = 1.0 / d.h;
+  d.Gd = (double)d.G;
+  d.ad = (double)d.a;
+  d.Hzd = (double)d.Hz;
+  d.theta2d = (double)d.theta2;
+  d.a_inv = 1.0 / (double)d.a;
+  d.hf = (float)d.h;
+  d.hinvf = (float)d.h_inv;
+  d.h2f = d.hf * d.hf;
   return d;
 }
 

@@ -48,31 +48,52 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 // Exact float -> double and round-to-nearest-even double -> float, built
 // from the IEEE-754 fields with integer operations: the conversion
 // instructions run on the FP64 unit, at 1/64 of the FP32 rate on this GPU.
-// Zero, subnormal, infinite and NaN inputs (and results outside the normal
-// float range) take the conversion instruction.
+// The special cases are integer code too.  A double instruction behind a
+// condition is no way out: the compiler predicates short branches, and a
+// predicated-off double instruction holds the FP64 unit as long as an executed
+// one (measured: 20 of them per step in a walk took it from 1.5 to 25 ms).
+// Rare double paths in this library are calls for the same reason.
 __device__ __forceinline__ double f2d(float x)
 {
-  const unsigned u = __float_as_uint(x);
+  unsigned u = __float_as_uint(x);
+  unsigned bias = 1023 - 127;
+  const unsigned sign = u & 0x80000000u;
   const unsigned e = (u >> 23) & 0xffu;
-  const unsigned long long s = (unsigned long long)(u >> 31) << 63;
-  if ((u & 0x7fffffffu) == 0u) return __longlong_as_double((long long)s);
-  if (e == 0u || e == 0xffu) return (double)x;
-  return __longlong_as_double((long long)(s | ((unsigned long long)(e + (1023 - 127)) << 52) |
-                                          ((unsigned long long)(u & 0x7fffffu) << 29)));
+  if (e == 0u) {  // zero or subnormal: 2^64 x is exact
+    u = __float_as_uint(__fmul_rn(x, 0x1p64f));
+    bias = (u & 0x7fffffffu) ? bias - 64 : 0;
+  }
+  if (e == 0xffu) bias = 0x7ff - 0xff;
+  const unsigned hi = sign | ((((u >> 23) & 0xffu) + bias) << 20) | ((u & 0x7fffffu) >> 3);
+  return __hiloint2double((int)hi, (int)(u << 29));
 }
 
 __device__ __forceinline__ float d2f(double x)
 {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int e = (int)((b >> 52) & 0x7ffull) - 1023 + 127;
-  if (e <= 0 || e >= 255) return __double2float_rn(x);
   const unsigned long long mant = b & 0xfffffffffffffull;
-  unsigned long long r = mant >> 29;
-  const unsigned long long rem = mant & 0x1fffffffull, half = 1ull << 28;
-  if (rem > half || (rem == half && (r & 1ull))) r++;
-  const unsigned bits = (unsigned)(((unsigned long long)e << 23) + r);  // a carry bumps the exponent
-  if (((bits >> 23) & 0xffu) == 0xffu) return __double2float_rn(x);
+  // round half to even; a carry bumps the exponent
+  unsigned bits = ((unsigned)e << 23) + (unsigned)(mant >> 29) +
+                  ((b & 0x1fffffffull) + ((mant >> 29) & 1ull) > (1ull << 28) ? 1u : 0u);
+  if (e <= 0) {  // a subnormal result, or zero
+    const int s = min(30 - e, 63);
+    const unsigned long long m = mant | (1ull << 52);
+    const unsigned long long q = m >> s, rem = m & ((1ull << s) - 1ull), half = 1ull << (s - 1);
+    bits = s > 53 ? 0u : (unsigned)q + (rem + (q & 1ull) > half ? 1u : 0u);
+  } else if (e >= 255 || bits >= 0x7f800000u) {  // overflow, infinity or NaN
+    bits = e == 0x7ff - 1023 + 127 && mant ? 0x7fc00000u : 0x7f800000u;
+  }
   return __uint_as_float(bits | ((unsigned)(b >> 63) << 31));
+}
+
+// x / 2, on the exponent where that is exact.
+__device__ __forceinline__ double half_of(double x)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned ex = (unsigned)(b >> 52) & 0x7ffu;
+  if (ex - 2u < 0x7ffu - 2u) return __longlong_as_double((long long)(b - (1ull << 52)));
+  return dmul(0.5, x);
 }
 
 // NEAREST (src/config_parser.h:142) on a double / a float operand.
@@ -111,6 +132,14 @@ __device__ __forceinline__ float vdot(const float a[3], const float b[3])
 // for |s| < box the wrap s -+ box is exact in float as in double (Sterbenz:
 // box/2 < |s| < 2 box), so the float arithmetic gives the same bits without
 // the FP64 pipe (1/64 of the FP32 rate on this GPU); otherwise the double path.
+static __device__ __noinline__ float rel_coord_double(float x, float c, int periodic, float box,
+                                                      float boxhalf)
+{
+  double d = dsub(f2d(x), f2d(c));
+  if (periodic) d = d > f2d(boxhalf) ? dsub(d, f2d(box)) : d < -f2d(boxhalf) ? dadd(d, f2d(box)) : d;
+  return d2f(d);
+}
+
 __device__ __forceinline__ float rel_coord(float x, float c, const DevParams &P)
 {
   const float s = __fsub_rn(x, c);
@@ -118,9 +147,7 @@ __device__ __forceinline__ float rel_coord(float x, float c, const DevParams &P)
   const float err = __fadd_rn(__fsub_rn(x, __fsub_rn(s, bb)), __fsub_rn(-c, bb));
   if (err == 0.f && !P.periodic) return s;
   if (err == 0.f && fabsf(s) < P.box) return nearest_f(s, P);
-  double d = dsub(f2d(x), f2d(c));
-  if (P.periodic) d = nearest_d(d, P);
-  return d2f(d);
+  return rel_coord_double(x, c, P.periodic, P.box, P.boxhalf);
 }
 
 // Order-preserving 32-bit key of a float (ascending); -0 sorts as +0.

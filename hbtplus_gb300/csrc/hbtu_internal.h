@@ -39,6 +39,9 @@ struct DevParams {
   int precision;
   long long maxsample;
   double h, h_inv;
+  double Gd, ad, Hzd, theta2d;  // G, a, Hz and theta2 as double
+  double a_inv;                 // 1 / a rounded to double
+  float hf, hinvf, h2f;         // h, 1 / h and hf * hf as floats (the FP32 walks')
 };
 
 DevParams derive_params(const hbtu_params &p);

@@ -538,13 +538,15 @@ __global__ void __launch_bounds__(kLB) k_avg_chunks(Ctx c)
 
 // ---------------------------------------------------------------- control
 // Sum k of subhalo s's chunks, in chunk order: one serial chain of double adds
-// (the order fixes the rounding), about 145 cycles each whatever runs ahead of
-// it (loads 16 at a time: no faster).
+// (the order fixes the rounding), about 145 cycles each (loads 16 ahead: no
+// faster).
 __device__ __forceinline__ double sum_chunks(const Ctx &c, int s, int k)
 {
+  const int b0 = c.bchunk_base[s], n = c.bchunk_base[s + 1] - b0;
+  const double *x = c.chunk_sums + (size_t)b0 * kSums + k;
   double t = 0.;
-  for (int b = c.bchunk_base[s]; b < c.bchunk_base[s + 1]; b++)
-    t += c.chunk_sums[(size_t)b * kSums + k];
+#pragma unroll 4
+  for (int b = 0; b < n; b++) t += x[(size_t)b * kSums];
   return t;
 }
 
@@ -671,56 +673,21 @@ __global__ void __launch_bounds__(kLB) k_kin_chunks(Ctx c)
   if (b >= c.bchunk_base[c.S]) return;
   const int s = upper_bound_i(c.bchunk_base, c.S + 1, b) - 1;
   const SegState &sg = c.seg[s];
-  const DevParams &P = c.P;
   const int nb = sg.nbound;
-  const int ci = b - c.bchunk_base[s];
-  const int lo = ci * kChunk, hi = min(lo + kChunk, nb);
-  double v[18];
-  for (int k = 0; k < 18; k++) v[k] = 0.;
-  int cnt[6] = {0, 0, 0, 0, 0, 0};
-  const double Pa = (double)P.a, PHz = (double)P.Hz;
-  for (int p = lo + threadIdx.x; p < hi; p += kLB) {
-    const int pid = c.epid[sg.off + p];
-    const float4 a = c.pm[pid], u = c.vel[pid];
-    const float m = a.w;
-    const float x[3] = {a.x, a.y, a.z}, w[3] = {u.x, u.y, u.z};
-    const double md = f2d(m);
-    v[0] += f2d(fmul(c.eE[sg.off + p], m));
-    double dx[3], dv[3];
-    for (int j = 0; j < 3; j++) {
-      // the wrap of a float difference below the box size is exact in float
-      // (Sterbenz), so it gives the double wrap's bits without the FP64 pipe
-      const float d = fsub(x[j], sg.ref_pos[j]);
-      if (!P.periodic)
-        dx[j] = f2d(d);
-      else if (fabsf(d) < P.box)
-        dx[j] = f2d(nearest_f(d, P));
-      else
-        dx[j] = nearest_d(f2d(d), P);
-      dx[j] = dmul(dx[j], Pa);
-      dv[j] = dadd(f2d(fsub(w[j], sg.ref_vel[j])), dmul(PHz, dx[j]));
-      v[1] += dmul(dmul(dv[j], dv[j]), md);
-    }
-    v[2] += dmul(dsub(dmul(dx[1], dv[2]), dmul(dx[2], dv[1])), md);
-    v[3] += dmul(dsub(dmul(dx[2], dv[0]), dmul(dx[0], dv[2])), md);
-    v[4] += dmul(dsub(dmul(dx[0], dv[1]), dmul(dx[1], dv[0])), md);
-    v[5] += md;
-    const int t = c.type ? c.type[pid] : 1;
-    const bool skip = (nb <= 100 && c.id[pid] == -1) || t < 0 || t > 5;
-    if (!skip) {
-      switch (t) {  // one double add per particle (the type is nearly always warp-uniform)
-        case 0: cnt[0]++; v[12] += md; break;
-        case 1: cnt[1]++; v[13] += md; break;
-        case 2: cnt[2]++; v[14] += md; break;
-        case 3: cnt[3]++; v[15] += md; break;
-        case 4: cnt[4]++; v[16] += md; break;
-        default: cnt[5]++; v[17] += md; break;
-      }
-    }
+  const int lo = (b - c.bchunk_base[s]) * kChunk, hi = min(lo + kChunk, nb);
+  // block_sum's sums: per warp, then the warps in order
+  __shared__ double sh[18][kLB / 32];
+  const int w = threadIdx.x >> 5;
+  if (32 * w < hi - lo)
+    kin_warp_sums(c, sg, nb, lo + threadIdx.x, hi, &sh[0][w], kLB / 32);
+  else if ((threadIdx.x & 31) < 18)
+    sh[threadIdx.x & 31][w] = 0.;
+  __syncthreads();
+  if (threadIdx.x < 18) {
+    double t = 0.;
+    for (int j = 0; j < kLB / 32; j++) t += sh[threadIdx.x][j];
+    c.chunk_sums[(size_t)b * kSums + threadIdx.x] = t;
   }
-#pragma unroll
-  for (int q = 0; q < 6; q++) v[6 + q] = (double)cnt[q];  // exact: counts < 2^53
-  block_sum<18>(v, c.chunk_sums + (size_t)b * kSums, hi - lo);
 }
 
 __global__ void k_final_seg(Ctx c, hbtu_result *res)
@@ -731,83 +698,9 @@ __global__ void k_final_seg(Ctx c, hbtu_result *res)
   const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= c.S) return;
   const SegState &sg = c.seg[s];
-  const DevParams &P = c.P;
   const bool summed = sg.status != SEG_TRIVIAL && sg.status != SEG_DISRUPTED;
   const double part = summed && lane < 18 ? sum_chunks(c, s, lane) : 0.;
-  double v[18];
-#pragma unroll
-  for (int k = 0; k < 18; k++) v[k] = __shfl_sync(0xffffffffu, part, k);
-  // the divisions by the mass, one per lane: E, 1/2 (for K), the angular momentum
-  const double num = lane == 0 ? v[0] : (lane == 1 ? 0.5 : (lane < 5 ? part : 1.));
-  const double quot = ddiv(num, summed && sg.nbound > 1 && lane < 5 ? v[5] : 1.);
-  double over_m[5];
-#pragma unroll
-  for (int k = 0; k < 5; k++) over_m[k] = __shfl_sync(0xffffffffu, quot, k);
-  if (lane != 0) return;
-  hbtu_result r;
-  memset(&r, 0, sizeof(r));
-  r.too_few = sg.n < P.minpart;
-  r.iterations = sg.passes;
-  r.evaluations = sg.evals;
-  r.interactions = sg.interactions;
-  for (int j = 0; j < 3; j++) {
-    r.ref_pos[j] = sg.ref_pos[j];
-    r.ref_vel[j] = sg.ref_vel[j];
-    r.mostbound_pos[j] = sg.mb_pos[j];
-    r.mostbound_vel[j] = sg.mb_vel[j];
-  }
-  if (sg.status == SEG_TRIVIAL) {  // src/subhalo_unbind.cpp:275-293 + CountParticles
-    r.nbound = sg.n;
-    if (sg.n == 1) {
-      const int t = c.type ? c.type[sg.off] : 1;
-      const float m = c.pm[sg.off].w;
-      if (t >= 0 && t <= 5) {
-        r.nbound_type[t] = 1;
-        r.mbound_type[t] = m;
-      }
-      float acc = 0.f;
-      for (int k = 0; k < 6; k++) acc = fadd(acc, r.mbound_type[k]);
-      r.mbound = acc;
-    }
-  } else if (sg.status == SEG_DISRUPTED) {
-    r.disrupted = 1;
-    r.nbound = 1;
-    r.mbound = sg.mbound;
-    const int k = sg.first_mb < sg.n ? sg.first_mb : 0;
-    const int t = c.type ? c.type[sg.off + k] : 1;
-    const bool skip = c.id[sg.off + k] == -1 || t < 0 || t > 5;
-    if (!skip) {
-      r.nbound_type[t] = 1;
-      r.mbound_type[t] = c.pm[sg.off + k].w;
-    }
-  } else {
-    r.converged = sg.status == SEG_CONVERGED;
-    if (sg.status == SEG_FAILED) r.status = HBTU_ERR_NOT_CONVERGED;
-    r.nbound = sg.nbound;
-    r.mbound = sg.mbound;
-    if (sg.nbound > 0) {
-      const int pid = c.epid[sg.off];
-      const float4 a = c.pm[pid], u = c.vel[pid];
-      r.mostbound_pos[0] = a.x;
-      r.mostbound_pos[1] = a.y;
-      r.mostbound_pos[2] = a.z;
-      r.mostbound_vel[0] = u.x;
-      r.mostbound_vel[1] = u.y;
-      r.mostbound_vel[2] = u.z;
-    }
-    if (sg.nbound > 1) {
-      const double E = over_m[0];
-      const double K = dmul(v[1], over_m[1]);
-      r.specific_potential = __double2float_rn(dsub(E, K));
-      r.specific_kinetic = __double2float_rn(K);
-      for (int j = 0; j < 3; j++) r.specific_angmom[j] = __double2float_rn(over_m[2 + j]);
-    }
-    for (int t = 0; t < 6; t++) {
-      r.nbound_type[t] = (int64_t)v[6 + t];
-      r.mbound_type[t] = (float)v[12 + t];
-    }
-  }
-  res[s] = r;
+  write_result(c, sg, part, lane, res + s);
 }
 
 __global__ void __launch_bounds__(kLB) k_final_out(Ctx c, int64_t *order, float *energy)
@@ -816,18 +709,7 @@ __global__ void __launch_bounds__(kLB) k_final_out(Ctx c, int64_t *order, float 
   const int p = blockIdx.x * kLB + threadIdx.x;
   if (p >= c.N) return;
   const SegState &sg = c.seg[c.pseg[p]];
-  const int l = p - sg.off;
-  if (sg.status == SEG_TRIVIAL) {
-    order[p] = l;
-    energy[p] = 0.f;
-  } else if (sg.status == SEG_DISRUPTED) {
-    const int k = sg.first_mb < sg.n ? sg.first_mb : 0;
-    order[p] = l == 0 ? k : (l == k ? 0 : l);
-    energy[p] = l == 0 ? sg.e0 : __int_as_float(0x7fc00000);
-  } else {
-    order[p] = c.epid[p] - sg.off;
-    energy[p] = c.eE[p];
-  }
+  write_position(c, sg, p, order, energy);
 }
 
 // Deterministic per-subhalo sums of x[off_s .. off_s + n_s): one block per

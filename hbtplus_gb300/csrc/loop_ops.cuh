@@ -37,6 +37,39 @@ __device__ __forceinline__ void rs_step(const double (&cur)[N], double (&nxt)[(N
   }
 }
 
+// A warp's sums of K values by that reduce-scatter: returns the index of the sum
+// this lane then holds in *sum, or -1.
+template <int K>
+__device__ __forceinline__ int warp_sums(const double (&v)[K], double *sum)
+{
+  static_assert(K >= 1 && K <= 32, "one sum per lane at most");
+  const int lane = threadIdx.x & 31;
+  constexpr int n1 = (K + 1) / 2, n2 = (n1 + 1) / 2, n3 = (n2 + 1) / 2, n4 = (n3 + 1) / 2,
+                n5 = (n4 + 1) / 2;
+  double a1[n1], a2[n2], a3[n3], a4[n4], a5[n5];
+  rs_step<K>(v, a1, 16, lane & 16);
+  rs_step<n1>(a1, a2, 8, lane & 8);
+  rs_step<n2>(a2, a3, 4, lane & 4);
+  rs_step<n3>(a3, a4, 2, lane & 2);
+  rs_step<n4>(a4, a5, 1, lane & 1);
+  // the index of the sum this lane holds: the split follows the padded
+  // sizes N; n counts the lane's real (unpadded) values
+  int base = 0, n = K, N = K;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const int h = (N + 1) / 2;
+    if (lane & o) {
+      base += h;
+      n = max(0, n - h);
+    } else {
+      n = min(n, h);
+    }
+    N = h;
+  }
+  *sum = a5[0];
+  return n >= 1 ? base : -1;
+}
+
 // Sums of K values over a block of kLB threads into out[0 .. K).  The
 // chunk's elements p = threadIdx.x + j*kLB (0 <= p < nvalid) are spread over
 // the warps in order, so a warp with 32*w >= nvalid holds only zeros and
@@ -44,33 +77,12 @@ __device__ __forceinline__ void rs_step(const double (&cur)[N], double (&nxt)[(N
 template <int K>
 __device__ void block_sum(double (&v)[K], double *out, int nvalid)
 {
-  static_assert(K >= 1 && K <= 32, "one sum per lane at most");
   __shared__ double sh[K][kLB / 32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (32 * w < nvalid) {
-    constexpr int n1 = (K + 1) / 2, n2 = (n1 + 1) / 2, n3 = (n2 + 1) / 2, n4 = (n3 + 1) / 2,
-                  n5 = (n4 + 1) / 2;
-    double a1[n1], a2[n2], a3[n3], a4[n4], a5[n5];
-    rs_step<K>(v, a1, 16, lane & 16);
-    rs_step<n1>(a1, a2, 8, lane & 8);
-    rs_step<n2>(a2, a3, 4, lane & 4);
-    rs_step<n3>(a3, a4, 2, lane & 2);
-    rs_step<n4>(a4, a5, 1, lane & 1);
-    // the index of the sum this lane holds: the split follows the padded
-    // sizes N; n counts the lane's real (unpadded) values
-    int base = 0, n = K, N = K;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int h = (N + 1) / 2;
-      if (lane & o) {
-        base += h;
-        n = max(0, n - h);
-      } else {
-        n = min(n, h);
-      }
-      N = h;
-    }
-    if (n >= 1) sh[base][w] = a5[0];
+    double sum;
+    const int k = warp_sums<K>(v, &sum);
+    if (k >= 0) sh[k][w] = sum;
   } else if (lane < K) {
     sh[lane][w] = 0.;
   }
@@ -90,6 +102,13 @@ __device__ void block_sum(double (&v)[K], double *out, int nvalid)
 // its fma remainder, added exactly in double: one FP64 add instead of the
 // double subtract, wrap and multiply (FP64 runs at 1/64 of the FP32 rate on
 // this GPU).  Otherwise the double path.
+static __device__ __noinline__ double rel_times_mass_double(float x, double od, double md,
+                                                            float box, float boxhalf)
+{
+  const double d = dsub(f2d(x), od);
+  return dmul(d > f2d(boxhalf) ? dsub(d, f2d(box)) : d < -f2d(boxhalf) ? dadd(d, f2d(box)) : d, md);
+}
+
 __device__ __forceinline__ double rel_times_mass(float x, float o, double od, float m, double md,
                                                  const DevParams &P)
 {
@@ -102,7 +121,7 @@ __device__ __forceinline__ double rel_times_mass(float x, float o, double od, fl
     const float r = __fmaf_rn(q, m, -p);  // q*m - p, exact
     return dadd(f2d(p), f2d(r));
   }
-  return dmul(nearest_d(dsub(f2d(x), od), P), md);
+  return rel_times_mass_double(x, od, md, P.box, P.boxhalf);
 }
 
 // One bound particle's terms of the frame sums: w[0] += m, w[1..3] += v*m
@@ -187,14 +206,14 @@ __device__ __forceinline__ void control_segment(const Ctx &c, SegState &sg, int 
     sg.ref_pos[1] = a.y;
     sg.ref_pos[2] = a.z;
   } else if (nb > 1) {
-    sg.mbound = (float)msum;
-    for (int j = 0; j < 3; j++) sg.ref_vel[j] = __double2float_rn(mean[j]);
+    sg.mbound = d2f(msum);
+    for (int j = 0; j < 3; j++) sg.ref_vel[j] = d2f(mean[j]);
     const float4 o = c.pm[c.epid[sg.off]];
-    const double org[3] = {o.x, o.y, o.z};
+    const double org[3] = {f2d(o.x), f2d(o.y), f2d(o.z)};
     for (int j = 0; j < 3; j++) {
       double x = mean[3 + j];
       if (P.periodic) x = dadd(x, org[j]);
-      sg.ref_pos[j] = __double2float_rn(x);
+      sg.ref_pos[j] = d2f(x);
     }
   } else {
     sg.mbound = 0.f;
@@ -213,7 +232,7 @@ __device__ __forceinline__ void control_segment(const Ctx &c, SegState &sg, int 
     sg.ntgt = nb;
     sg.mfac = 1.f;
     relvel(sg.old_pos, sg.old_vel, sg.ref_pos, sg.ref_vel, sg.dV, P);
-    sg.dK = __double2float_rn(dmul(0.5, (double)vdot(sg.dV, sg.dV)));
+    sg.dK = d2f(half_of(f2d(vdot(sg.dV, sg.dV))));
     sg.tgt_mode = sg.coh_n > 0 ? 1 : 2;
   } else {  // full pass (:331-356)
     sg.mode = MODE_FULL;
@@ -231,6 +250,206 @@ __device__ __forceinline__ void control_segment(const Ctx &c, SegState &sg, int 
   }
   sg.nlast = nb;
   if (sg.passes >= max_passes) sg.status = SEG_FAILED;
+}
+
+static __device__ __noinline__ double nearest_double(double x, float box, float boxhalf)
+{
+  return x > f2d(boxhalf) ? dsub(x, f2d(box)) : x < -f2d(boxhalf) ? dadd(x, f2d(box)) : x;
+}
+
+// Type of bound particle pid for the per-type sums, -1: not counted
+// (CountParticleTypes, src/subhalo.cpp:400-444); nb: Nbound.
+__device__ __forceinline__ int counted_type(const Ctx &c, int nb, int pid)
+{
+  const int t = c.type ? c.type[pid] : 1;
+  return (nb <= 100 && c.id[pid] == -1) || t < 0 || t > 5 ? -1 : t;
+}
+
+// One bound particle's terms of the final sums (list position p of nb):
+// binding energy, kinetic energy, angular momentum and mass (AverageKinematics,
+// src/subhalo_unbind.cpp:189-232).
+__device__ __forceinline__ void kin_terms(const Ctx &c, const SegState &sg, int pid, float E,
+                                          double (&v)[7])
+{
+  const DevParams &P = c.P;
+  const float4 a = c.pm[pid], u = c.vel[pid];
+  const float m = a.w;
+  const float x[3] = {a.x, a.y, a.z}, w[3] = {u.x, u.y, u.z};
+  const double md = f2d(m);
+  v[0] += f2d(fmul(E, m));
+  double dx[3], dv[3];
+  for (int j = 0; j < 3; j++) {
+    // the wrap of a float difference below the box size is exact in float
+    // (Sterbenz), so it gives the double wrap's bits without the FP64 pipe
+    const float d = fsub(x[j], sg.ref_pos[j]);
+    if (!P.periodic)
+      dx[j] = f2d(d);
+    else if (fabsf(d) < P.box)
+      dx[j] = f2d(nearest_f(d, P));
+    else
+      dx[j] = nearest_double(f2d(d), P.box, P.boxhalf);
+    dx[j] = dmul(dx[j], P.ad);
+    dv[j] = dadd(f2d(fsub(w[j], sg.ref_vel[j])), dmul(P.Hzd, dx[j]));
+    v[1] += dmul(dmul(dv[j], dv[j]), md);
+  }
+  v[2] += dmul(dsub(dmul(dx[1], dv[2]), dmul(dx[2], dv[1])), md);
+  v[3] += dmul(dsub(dmul(dx[2], dv[0]), dmul(dx[0], dv[2])), md);
+  v[4] += dmul(dsub(dmul(dx[0], dv[1]), dmul(dx[1], dv[0])), md);
+  v[5] += md;
+}
+
+// A warp's final sums over the list positions first, first + kLB, ... < hi of each
+// lane (Nbound nb), in the association of block_sum<18>: sums 0..5 are
+// kin_terms', 6..11 the counts of each type and 12..17 their masses; sum k to
+// out[k * stride].  Almost always a warp's particles are of one type: then five of
+// the masses' sums are zero, and seven sums are reduced instead of 18.
+__device__ __forceinline__ void kin_warp_sums(const Ctx &c, const SegState &sg, int nb, int first,
+                                              int hi, double *out, int stride)
+{
+  const int lane = threadIdx.x & 31;
+  double v[7] = {0., 0., 0., 0., 0., 0., 0.};
+  int cnt[6] = {0, 0, 0, 0, 0, 0};
+  int lo_t = 6, hi_t = -1;  // the types met
+  for (int p = first; p < hi; p += kLB) {
+    const int pid = c.epid[sg.off + p];
+    kin_terms(c, sg, pid, c.eE[sg.off + p], v);
+    const int t = counted_type(c, nb, pid);
+    if (t >= 0) {
+      lo_t = min(lo_t, t);
+      hi_t = max(hi_t, t);
+      v[6] += f2d(c.pm[pid].w);
+    }
+#pragma unroll
+    for (int q = 0; q < 6; q++) cnt[q] += t == q;
+  }
+  const int t0 = __reduce_min_sync(0xffffffffu, lo_t), t1 = __reduce_max_sync(0xffffffffu, hi_t);
+  double sum;
+  const int k = warp_sums<7>(v, &sum);
+  if (k >= 0 && k < 6) out[k * stride] = sum;
+#pragma unroll
+  for (int q = 0; q < 6; q++) cnt[q] = __reduce_add_sync(0xffffffffu, cnt[q]);
+  if (lane < 6) {
+    int n = cnt[0];
+#pragma unroll
+    for (int q = 1; q < 6; q++) n = lane == q ? cnt[q] : n;
+    out[(6 + lane) * stride] = (double)n;  // exact
+    if (t0 >= t1 && lane != t0) out[(12 + lane) * stride] = 0.;
+  }
+  if (t0 >= t1) {
+    if (k == 6 && t1 >= 0) out[(12 + t0) * stride] = sum;
+    return;
+  }
+  double w[6] = {0., 0., 0., 0., 0., 0.};  // several types
+  for (int p = first; p < hi; p += kLB) {
+    const int pid = c.epid[sg.off + p];
+    const int t = counted_type(c, nb, pid);
+    const double md = f2d(c.pm[pid].w);
+#pragma unroll
+    for (int q = 0; q < 6; q++) w[q] += t == q ? md : 0.;
+  }
+  const int q = warp_sums<6>(w, &sum);
+  if (q >= 0) out[(12 + q) * stride] = sum;
+}
+
+// A subhalo's result record, by one warp: lanes 0..17 hold the sums of
+// kin_terms (v[6..11] the type counts) when it is neither trivial nor disrupted.
+__device__ __forceinline__ void write_result(const Ctx &c, const SegState &sg, double part,
+                                             int lane, hbtu_result *res)
+{
+  const DevParams &P = c.P;
+  const bool summed = sg.status != SEG_TRIVIAL && sg.status != SEG_DISRUPTED;
+  double v[18];
+#pragma unroll
+  for (int k = 0; k < 18; k++) v[k] = __shfl_sync(0xffffffffu, part, k);
+  // the divisions by the mass, one per lane: E, 1/2 (for K), the angular momentum
+  const double num = lane == 0 ? v[0] : (lane == 1 ? 0.5 : (lane < 5 ? part : 1.));
+  const double quot = ddiv(num, summed && sg.nbound > 1 && lane < 5 ? v[5] : 1.);
+  double over_m[5];
+#pragma unroll
+  for (int k = 0; k < 5; k++) over_m[k] = __shfl_sync(0xffffffffu, quot, k);
+  if (lane != 0) return;
+  hbtu_result r;
+  memset(&r, 0, sizeof(r));
+  r.too_few = sg.n < P.minpart;
+  r.iterations = sg.passes;
+  r.evaluations = sg.evals;
+  r.interactions = sg.interactions;
+  for (int j = 0; j < 3; j++) {
+    r.ref_pos[j] = sg.ref_pos[j];
+    r.ref_vel[j] = sg.ref_vel[j];
+    r.mostbound_pos[j] = sg.mb_pos[j];
+    r.mostbound_vel[j] = sg.mb_vel[j];
+  }
+  if (sg.status == SEG_TRIVIAL) {  // src/subhalo_unbind.cpp:275-293 + CountParticles
+    r.nbound = sg.n;
+    if (sg.n == 1) {
+      const int t = c.type ? c.type[sg.off] : 1;
+      const float m = c.pm[sg.off].w;
+      if (t >= 0 && t <= 5) {
+        r.nbound_type[t] = 1;
+        r.mbound_type[t] = m;
+      }
+      float acc = 0.f;
+      for (int k = 0; k < 6; k++) acc = fadd(acc, r.mbound_type[k]);
+      r.mbound = acc;
+    }
+  } else if (sg.status == SEG_DISRUPTED) {
+    r.disrupted = 1;
+    r.nbound = 1;
+    r.mbound = sg.mbound;
+    const int k = sg.first_mb < sg.n ? sg.first_mb : 0;
+    const int t = c.type ? c.type[sg.off + k] : 1;
+    const bool skip = c.id[sg.off + k] == -1 || t < 0 || t > 5;
+    if (!skip) {
+      r.nbound_type[t] = 1;
+      r.mbound_type[t] = c.pm[sg.off + k].w;
+    }
+  } else {
+    r.converged = sg.status == SEG_CONVERGED;
+    if (sg.status == SEG_FAILED) r.status = HBTU_ERR_NOT_CONVERGED;
+    r.nbound = sg.nbound;
+    r.mbound = sg.mbound;
+    if (sg.nbound > 0) {
+      const int pid = c.epid[sg.off];
+      const float4 a = c.pm[pid], u = c.vel[pid];
+      r.mostbound_pos[0] = a.x;
+      r.mostbound_pos[1] = a.y;
+      r.mostbound_pos[2] = a.z;
+      r.mostbound_vel[0] = u.x;
+      r.mostbound_vel[1] = u.y;
+      r.mostbound_vel[2] = u.z;
+    }
+    if (sg.nbound > 1) {
+      const double E = over_m[0];
+      const double K = dmul(v[1], over_m[1]);
+      r.specific_potential = d2f(dsub(E, K));
+      r.specific_kinetic = d2f(K);
+      for (int j = 0; j < 3; j++) r.specific_angmom[j] = d2f(over_m[2 + j]);
+    }
+    for (int t = 0; t < 6; t++) {
+      r.nbound_type[t] = (int64_t)v[6 + t];
+      r.mbound_type[t] = d2f(v[12 + t]);
+    }
+  }
+  *res = r;
+}
+
+// Order and energy at global list position p of subhalo sg.
+__device__ __forceinline__ void write_position(const Ctx &c, const SegState &sg, int p,
+                                               int64_t *order, float *energy)
+{
+  const int l = p - sg.off;
+  if (sg.status == SEG_TRIVIAL) {
+    order[p] = l;
+    energy[p] = 0.f;
+  } else if (sg.status == SEG_DISRUPTED) {
+    const int k = sg.first_mb < sg.n ? sg.first_mb : 0;
+    order[p] = l == 0 ? k : (l == k ? 0 : l);
+    energy[p] = l == 0 ? sg.e0 : __int_as_float(0x7fc00000);
+  } else {
+    order[p] = c.epid[p] - sg.off;
+    energy[p] = c.eE[p];
+  }
 }
 
 }  // namespace hbtu

@@ -290,10 +290,10 @@ __device__ void walk_targets(const Ctx &c, int s, SegState &sg, int P0, const in
       }
     }
     Target t;
-    init_target<!kFP64>(c, s, epos, pid, active, 2 * P0, t);
+    init_target<!kFP64>(c, sg, s, epos, pid, active, 2 * P0, t);
     int ninter = 0;
-    const double pot = kFP64 ? walk_fp64(c, t, &ninter) : walk_lean<false>(c.nd, t, c.P, &ninter);
-    finish_target(c, t, pot);
+    const double pot = kFP64 ? walk_fp64(c, t, &ninter) : walk_lean<false, true>(c.nd, t, c.P, &ninter);
+    finish_target(c, sg, t, pot);
     count_interactions(c, s, ninter);
   }
   __syncthreads();

@@ -101,15 +101,6 @@ __device__ __forceinline__ bool float_fixed(float x, int E, long long &X)
   return true;
 }
 
-// x / 2, on the exponent where that is exact.
-__device__ __forceinline__ double half_of(double x)
-{
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned ex = (unsigned)(b >> 52) & 0x7ffu;
-  if (ex - 2u < 0x7ffu - 2u) return __longlong_as_double((long long)(b - (1ull << 52)));
-  return dmul(0.5, x);
-}
-
 // Depth of geometric subdivision of a cube of side len: the number of
 // halvings until the side is below res (the len halving rule of
 // src/gravity_tree.cpp:37-40), at most kMaxLevels, from exponents and mantissas.
@@ -410,6 +401,11 @@ __device__ __forceinline__ double recip_refined(double m, bool &ok)
 // equal masses takes 12 to 15 double operations in all, where the
 // division's own (per axis, for the whole warp when one lane needs it)
 // more than doubled that: double runs at 1/64 of the FP32 rate on this GPU.
+static __device__ __noinline__ float quot_float_divided(double c, double m)
+{
+  return d2f(ddiv(c, m));
+}
+
 __device__ __forceinline__ float quot_float(double c, double m, double r, bool ok)
 {
   const double q = dmul(c, r);
@@ -433,7 +429,7 @@ __device__ __forceinline__ float quot_float(double c, double m, double r, bool o
       return __uint_as_float(bits | ((unsigned)(mid >> 63) << 31));
     }
   }
-  return d2f(ddiv(c, m));
+  return quot_float_divided(c, m);
 }
 
 // Bottom-up moments of one cell: mass and centre of mass over its children in
@@ -451,8 +447,7 @@ __device__ __forceinline__ float4 cell_moment_slots(bool bucket, int idx, int en
                                                     int4 s1, Src src)
 {
   double m = 0., cx = 0., cy = 0., cz = 0.;
-  auto add = [&](int k) {
-    const float4 a = src(k);
+  auto add = [&](float4 a) {
     const double w = f2d(a.w);
     m = dadd(m, w);
     cx = __fma_rn(f2d(a.x), w, cx);
@@ -461,21 +456,30 @@ __device__ __forceinline__ float4 cell_moment_slots(bool bucket, int idx, int en
   };
   if (!bucket) {
     // the occupied octants in ascending order; a warp then issues as many
-    // (double) additions as its lanes' largest number of children, not eight
+    // (double) additions as its lanes' largest number of children, not eight.
+    // Two at a time, so that both moments are on their way before the first
+    // is added.
     const int sl[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
     unsigned occ = 0;
 #pragma unroll
     for (int j = 0; j < 8; j++) occ |= (sl[j] > idx && sl[j] < end ? 1u : 0u) << j;
-    while (occ) {
+    auto take = [&]() {
       const int j = __ffs(occ) - 1;
       occ &= occ - 1;
       const int4 h = j < 4 ? s0 : s1;
       const int q = j & 3;
-      add(q == 0 ? h.x : (q == 1 ? h.y : (q == 2 ? h.z : h.w)));
+      return q == 0 ? h.x : (q == 1 ? h.y : (q == 2 ? h.z : h.w));
+    };
+    while (occ) {
+      const int k0 = take();
+      const int k1 = occ ? take() : -1;
+      const float4 a0 = src(k0), a1 = src(k1 >= 0 ? k1 : k0);
+      add(a0);
+      if (k1 >= 0) add(a1);
     }
   } else {
 #pragma unroll 4
-    for (int k = idx + 1; k < end; k++) add(k);
+    for (int k = idx + 1; k < end; k++) add(src(k));
   }
   bool ok;
   const double r = recip_refined(m, ok);

@@ -67,7 +67,7 @@ __device__ __forceinline__ void load_target(const Ctx &c, int w, int total, Targ
     pid = c.epid[epos];
     active = true;
   }
-  init_target<kRel>(c, s, epos, pid, active, 2 * c.tree_base[s], t);
+  init_target<kRel>(c, sg, s, epos, pid, active, 2 * c.tree_base[s], t);
 }
 
 // FP32 walk, warp schedule.  Leaf runs: when targets open a cell
@@ -84,8 +84,8 @@ __global__ void __launch_bounds__(kWB) k_walk_fp32(Ctx c, int total)
   load_target<true>(c, blockIdx.x * kWB + threadIdx.x, total, t);
   PotAcc acc;
   const float theta2 = P.theta2;
-  const float hf = (float)P.h, hinvf = (float)P.h_inv, h2f = hf * hf;
-  const double th2d = (double)P.theta2;
+  const float hf = P.hf, hinvf = P.hinvf, h2f = P.h2f;
+  const double th2d = P.theta2d;
   int ninter = 0;
   unsigned steps = 0;
 
@@ -154,20 +154,20 @@ __global__ void __launch_bounds__(kWB) k_walk_fp32(Ctx c, int total)
     }
     if ((++steps & 7u) == 0u) acc.flush();
   }
-  finish_target(c, t, acc.total((double)__fdiv_rn(t.mself, P.eps)));  // + cancels the self term
+  finish_target(c, c.seg[t.s], t, acc.total((double)__fdiv_rn(t.mself, P.eps)));  // + cancels the self term
   count_interactions(c, t.s, ninter);
 }
 
 // FP32 walk, lane schedule (walk_lean): blocks of kB neighbouring targets.
-template <int kB, bool kSib>
+template <int kB, bool kSib, bool kFlat>
 __global__ void __launch_bounds__(kB) k_walk_fp32_lean(Ctx c, int total)
 {
   HBTU_KERNEL_PROLOGUE();
   Target t;
   load_target<true>(c, blockIdx.x * kB + threadIdx.x, total, t);
   int ninter = 0;
-  const double pot = walk_lean<kSib>(kSib ? c.nd2 : c.nd, t, c.P, &ninter);
-  finish_target(c, t, pot);
+  const double pot = walk_lean<kSib, kFlat>(kSib ? c.nd2 : c.nd, t, c.P, &ninter);
+  finish_target(c, c.seg[t.s], t, pot);
   count_interactions(c, t.s, ninter);
 }
 
@@ -175,11 +175,11 @@ template <bool kSib>
 void launch_lean(Ctx &c, int n)
 {
   if (n >= 152 * 4 * 512)  // blocks of neighbouring targets share an SM's L1
-    launch_k(k_walk_fp32_lean<512, kSib>, (n + 511) / 512, 512, 0, c.st, c, n);
+    launch_k(k_walk_fp32_lean<512, kSib, false>, (n + 511) / 512, 512, 0, c.st, c, n);
   else if (n >= 152 * 4 * 256)
-    launch_k(k_walk_fp32_lean<256, kSib>, (n + 255) / 256, 256, 0, c.st, c, n);
+    launch_k(k_walk_fp32_lean<256, kSib, true>, (n + 255) / 256, 256, 0, c.st, c, n);
   else
-    launch_k(k_walk_fp32_lean<128, kSib>, (n + 127) / 128, 128, 0, c.st, c, n);
+    launch_k(k_walk_fp32_lean<128, kSib, true>, (n + 127) / 128, 128, 0, c.st, c, n);
 }
 
 // FP64: the reference's arithmetic, operation by operation (walk_fp64), one
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kWB) k_walk_fp64(Ctx c, int total)
   load_target<false>(c, blockIdx.x * kWB + threadIdx.x, total, t);
   int ninter = 0;
   const double pot = walk_fp64(c, t, &ninter);
-  finish_target(c, t, pot);
+  finish_target(c, c.seg[t.s], t, pot);
   count_interactions(c, t.s, ninter);
 }
 
@@ -227,8 +227,8 @@ template <bool kSib, bool kGrad>
 __device__ __forceinline__ double walk_grad(const WNode *nodes, const Target &t,
                                             const DevParams &P, double (&acc)[3])
 {
-  const float hf = (float)P.h, hinvf = (float)P.h_inv, h2f = hf * hf;
-  const double th2d = (double)P.theta2;
+  const float hf = P.hf, hinvf = P.hinvf, h2f = P.h2f;
+  const double th2d = P.theta2d;
   float hi = 0.f, comp = 0.f;  // Kahan sum of the potential
   // compensated (Kahan) float sums of the gradient: no double arithmetic in the
   // loop, where the lanes of a warp drift apart and a double instruction would

@@ -25,10 +25,9 @@ struct Target {
 // absolute), the self term it cancels (full and refine passes, if it is in
 // the tree), and the node range of the subhalo's tree.
 template <bool kRel>
-__device__ __forceinline__ void init_target(const Ctx &c, int s, int epos, int pid, bool active,
-                                            int root, Target &t)
+__device__ __forceinline__ void init_target(const Ctx &c, const SegState &sg, int s, int epos,
+                                            int pid, bool active, int root, Target &t)
 {
-  const SegState &sg = c.seg[s];
   t.s = s;
   t.epos = epos;
   t.pid = pid;
@@ -54,25 +53,40 @@ __device__ __forceinline__ void init_target(const Ctx &c, int s, int epos, int p
   t.nxt = nn > 0 ? root : kDone;
 }
 
+// x / a for the scale factor a, correctly rounded: a quotient from the
+// rounded reciprocal, corrected twice by its exact remainder (Markstein 1990:
+// the first correction brings it within a unit in the last place, the second
+// rounds it correctly).  Five double operations; a quotient or remainder that
+// could leave the normal range takes the division.
+__device__ __forceinline__ double over_scale(double x, const DevParams &P)
+{
+  if (P.a == 1.f) return x;
+  const unsigned ex = (unsigned)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu;
+  if (ex - 200u > 1600u) return ddiv(x, P.ad);
+  double q = dmul(x, P.a_inv);
+  q = __fma_rn(__fma_rn(-P.ad, q, x), P.a_inv, q);
+  return __fma_rn(__fma_rn(-P.ad, q, x), P.a_inv, q);
+}
+
 // BindingEnergy (full pass) or the correction update, and the store.
-__device__ __forceinline__ void finish_target(const Ctx &c, const Target &t, double pot_sum)
+__device__ __forceinline__ void finish_target(const Ctx &c, const SegState &sg, const Target &t,
+                                              double pot_sum)
 {
   if (!t.active) return;
   const DevParams &P = c.P;
-  const SegState &sg = c.seg[t.s];
-  const double pot = ddiv(dmul(pot_sum, (double)P.G), (double)P.a);
+  const double pot = over_scale(dmul(pot_sum, P.Gd), P);
   const float4 a = c.pm[t.pid], v = c.vel[t.pid];
   const float tp[3] = {a.x, a.y, a.z}, tv[3] = {v.x, v.y, v.z};
   float E;
   if (sg.mode != MODE_CORRECTION) {
     float dv[3];
     relvel(tp, tv, sg.ref_pos, sg.ref_vel, dv, P);
-    E = __double2float_rn(dadd(dmul((double)vdot(dv, dv), 0.5), pot));
+    E = d2f(dadd(half_of(f2d(vdot(dv, dv))), pot));
   } else {
     float ov[3];
     relvel(tp, tv, sg.old_pos, sg.old_vel, ov, P);
     const float tt = fadd(vdot(ov, sg.dV), sg.dK);
-    E = __double2float_rn(dadd((double)c.eE[t.epos], dsub((double)tt, pot)));
+    E = d2f(dadd(f2d(c.eE[t.epos]), dsub(f2d(tt), pot)));
   }
   if (sg.mode == MODE_REFINE)
     c.eR[t.epos] = E;
@@ -167,17 +181,16 @@ __device__ __forceinline__ void interact(float4 na, float r2, float &pot_f, floa
 }
 
 // The reference's opening decision in double, for a target whose float test
-// fell within 1e-5 of the threshold.  Not inlined: the compiler would
-// otherwise evaluate the double arithmetic on every step and select.
-// The target position comes by value, so the walk keeps it in registers.
+// fell within 1e-5 of the threshold: a call, so that a walk's steps issue no
+// double instruction otherwise.
 static __device__ __noinline__ bool exact_open(float4 na, float qx, float qy, float qz, float l2,
-                                        double th2d)
+                                               double th2d)
 {
-  const double ex = dsub((double)na.x, (double)qx);
-  const double ey = dsub((double)na.y, (double)qy);
-  const double ez = dsub((double)na.z, (double)qz);
+  const double ex = dsub(f2d(na.x), f2d(qx));
+  const double ey = dsub(f2d(na.y), f2d(qy));
+  const double ez = dsub(f2d(na.z), f2d(qz));
   const double er2 = dadd(dadd(dmul(ex, ex), dmul(ey, ey)), dmul(ez, ez));
-  return (double)l2 > dmul(er2, th2d);
+  return f2d(l2) > dmul(er2, th2d);
 }
 
 // FP32 walk of one target, lane schedule: the opening test is two compares
@@ -186,70 +199,110 @@ static __device__ __noinline__ bool exact_open(float4 na, float qx, float qy, fl
 // interaction goes straight into a compensated float sum, and the walk ends
 // when the index leaves the tree (skip pointers that leave it are kDone).
 //   kSib = false: preorder records; the next node is cur + 1 on opening, the
-//     skip pointer otherwise, so the index strictly grows and the loop ends
-//     even on a malformed tree.
+//     skip pointer otherwise.
 //   kSib = true: the sibling-block records (nd2): a cell's children sit in
 //     consecutive slots, so the sibling an accepted cell hands on to is
 //     usually in the same cache line; the next node is the first-child
-//     pointer (m.w) on opening and the skip pointer otherwise, the upper
-//     threshold is recomputed from the lower one, and the loop also stops
-//     after as many steps as the tree has nodes.  Same nodes, same order,
+//     pointer (m.w) on opening and the skip pointer otherwise, and the upper
+//     threshold is recomputed from the lower one.  Same nodes, same order,
 //     same sums as the preorder walk.
+// Both stop after as many steps as the tree has nodes, whatever its pointers.
+//
+// A step's chain is load, distance, decision, next load; the interaction hangs
+// off it.  The next node's load is therefore issued as soon as the decision is
+// known, before the interaction is computed.  With few targets the chip waits on
+// that chain, and kFlat keeps the interaction from stretching it: the softened
+// potential is computed on every step and selected, without a branch that the
+// lanes of a warp take apart (first pass of a 1.1e5-particle subhalo: 925 -> 657
+// us, 5e4 particles 732 -> 474 us).  With many targets the instructions count, and
+// the branch is the better form (867,289 targets: 2 to 4% faster than kFlat).
+// Two targets per lane over the union of their walks (1.18 nodes per node of one)
+// took 41% of the loads away but not the time: 92 instructions a step against
+// 2 x 49, at lower occupancy.
 // Returns the potential sum (self term cancelled, before G/a); *ninter counts
 // the interactions.
 constexpr float kBandRatio = 1.0000200002f;  // (1 + 1e-5) / (1 - 1e-5), rounded up
 
-template <bool kSib>
+// 1/sqrt(x) for x >= 1e-30: without the subnormal inputs' scaling, which such an
+// x never needs, the result is rsqrtf's.
+__device__ __forceinline__ float rsqrt_normal(float x)
+{
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// softened_fp32 without a branch: both polynomials (the fused multiply-adds
+// that softened_fp32 contracts to), then one is taken.
+__device__ __forceinline__ float softened_select(float m, float r2, float rinv, float hf,
+                                                 float hinvf)
+{
+  const float u = __fmul_rn(__fmul_rn(r2, rinv), hinvf);
+  const float uu = __fmul_rn(u, u);
+  const float in = __fmaf_rn(
+      uu, __fmaf_rn(uu, __fmaf_rn(6.4f, u, -9.6f), 5.333333333333f), -2.8f);
+  const float out = __fmaf_rn(
+      uu,
+      __fmaf_rn(u, __fmaf_rn(u, __fmaf_rn(-2.133333333333f, u, 9.6f), -16.0f), 10.666666666667f),
+      __fmaf_rn(0.066666666667f, __fmul_rn(hf, rinv), -3.2f));
+  return __fmul_rn(__fmul_rn(m, hinvf), u < 0.5f ? in : out);
+}
+
+template <bool kSib, bool kFlat>
 __device__ __forceinline__ double walk_lean(const WNode *nodes, const Target &t,
                                             const DevParams &P, int *ninter)
 {
-  const float hf = (float)P.h, hinvf = (float)P.h_inv, h2f = hf * hf;
-  const double th2d = (double)P.theta2;
+  const float hf = P.hf, hinvf = P.hinvf, h2f = P.h2f;
   float hi = 0.f, comp = 0.f;  // Kahan sum
-  int iters = 0, nopen = 0;
-  int cur = t.nxt;
-  const int end = t.end;
-  const int steps = kSib ? max(end - t.nxt, 0) : 0;  // the tree's node count
-  while (cur < end) {
+  int nacc = 0;
+  const int root = t.nxt;
+  const unsigned nn = t.end > root ? (unsigned)(t.end - root) : 0u;
+  if (nn > 0u) {
+    unsigned left = nn;  // steps left
+    int cur = root;
     float4 na;
     int4 nm;
     load_node(nodes, cur, na, nm);
-    const float r2 = dist2(na, t.q);
-    const float lo = __int_as_float(nm.z);
-    const float up = kSib ? lo * kBandRatio : __int_as_float(nm.w);
-    bool open = r2 < lo;
-    if (r2 >= lo && r2 <= up)
-      open = exact_open(na, t.q[0], t.q[1], t.q[2], __int_as_float(nm.x & 0x7fffffff), th2d);
-    const float rinv = rsqrtf(fmaxf(r2, 1e-30f));
-    const float mass = fabsf(na.w);
-    float contrib = -mass * rinv;
-    if (r2 < h2f) contrib = softened_fp32(mass, r2, rinv, hf, hinvf);
-    contrib = open ? 0.f : contrib;
-    const float y = __fsub_rn(contrib, comp);
-    const float s = __fadd_rn(hi, y);
-    comp = __fsub_rn(__fsub_rn(s, hi), y);
-    hi = s;
-    iters++;
-    nopen += open ? 1 : 0;
-    if (kSib) {
-      cur = open ? nm.w : nm.y;
-      if (iters >= steps || cur < t.nxt) break;  // malformed pointers: stop
-    } else {
-      cur = open ? cur + 1 : max(nm.y, cur + 1);
-    }
+    bool go;
+    do {
+      const float r2 = dist2(na, t.q);
+      const float lo = __int_as_float(nm.z);
+      const float up = kSib ? lo * kBandRatio : __int_as_float(nm.w);
+      bool open = r2 < lo;
+      if (r2 >= lo && r2 <= up)
+        open = exact_open(na, t.q[0], t.q[1], t.q[2], __int_as_float(nm.x & 0x7fffffff),
+                          P.theta2d);
+      const int next = open ? (kSib ? nm.w : cur + 1) : nm.y;
+      go = --left > 0u && (unsigned)(next - root) < nn;
+      cur = go ? next : root;  // the last load is not used
+      const float mass = fabsf(na.w);
+      load_node(nodes, cur, na, nm);
+      const float rinv = rsqrt_normal(fmaxf(r2, 1e-30f));
+      float contrib = __fmul_rn(-mass, rinv);
+      if (kFlat) {
+        const float near = softened_select(mass, r2, rinv, hf, hinvf);
+        contrib = r2 < h2f ? near : contrib;
+      } else if (r2 < h2f) {
+        contrib = softened_fp32(mass, r2, rinv, hf, hinvf);
+      }
+      // an opened node adds zero, which can still settle the compensation
+      const float y = __fsub_rn(open ? 0.f : contrib, comp);
+      const float s = __fadd_rn(hi, y);
+      comp = __fsub_rn(__fsub_rn(s, hi), y);
+      hi = s;
+      nacc += open ? 0 : 1;
+    } while (go);
   }
-  *ninter = iters - nopen;
-  const double base = (double)__fdiv_rn(t.mself, P.eps);  // cancels the self term
-  return dadd(dadd(base, (double)hi), -(double)comp);
+  *ninter = nacc;
+  const double base = f2d(__fdiv_rn(t.mself, P.eps));  // cancels the self term
+  return dadd(dadd(base, f2d(hi)), -f2d(comp));
 }
 
 // One FP64 interaction with the reference's arithmetic, operation by operation
 // (src/gravity_tree.cpp:136-160).
-__device__ __forceinline__ double fp64_contrib(double r2, double mass, const DevParams &P)
+static __device__ __noinline__ double fp64_softened(double r, double mass, double h_inv)
 {
-  const double r = __dsqrt_rn(r2);
-  if (r >= P.h) return -ddiv(mass, r);
-  const double u = dmul(r, P.h_inv);
+  const double u = dmul(r, h_inv);
   const double uu = dmul(u, u);
   double wp;
   if (u < 0.5)
@@ -258,7 +311,14 @@ __device__ __forceinline__ double fp64_contrib(double r2, double mass, const Dev
     wp = dadd(dadd(-3.2, ddiv(0.066666666667, u)),
               dmul(uu, dadd(10.666666666667,
                             dmul(u, dadd(-16.0, dmul(u, dsub(9.6, dmul(2.133333333333, u))))))));
-  return dmul(dmul(mass, P.h_inv), wp);
+  return dmul(dmul(mass, h_inv), wp);
+}
+
+__device__ __forceinline__ double fp64_contrib(double r2, double mass, const DevParams &P)
+{
+  const double r = __dsqrt_rn(r2);
+  if (r >= P.h) return -ddiv(mass, r);
+  return fp64_softened(r, mass, P.h_inv);
 }
 
 // FP64 walk of one target, lane schedule, over the preorder records: absolute
@@ -271,6 +331,14 @@ __device__ __forceinline__ double fp64_contrib(double r2, double mass, const Dev
 // |s| < box its wrap is exact in float as well (Sterbenz), so the double pipe
 // (1/64 of the FP32 rate on this GPU) only converts the result; otherwise the
 // double path.
+static __device__ __noinline__ double sep_fp64_double(float x, float q, int periodic, float box,
+                                                      float boxhalf)
+{
+  const double d = dsub(f2d(x), f2d(q));
+  if (!periodic) return d;
+  return d > f2d(boxhalf) ? dsub(d, f2d(box)) : d < -f2d(boxhalf) ? dadd(d, f2d(box)) : d;
+}
+
 __device__ __forceinline__ double sep_fp64(float x, float q, const DevParams &P)
 {
   const float s = __fsub_rn(x, q);
@@ -278,15 +346,14 @@ __device__ __forceinline__ double sep_fp64(float x, float q, const DevParams &P)
   const float err = __fadd_rn(__fsub_rn(x, __fsub_rn(s, bb)), __fsub_rn(-q, bb));
   if (err == 0.f && !P.periodic) return f2d(s);
   if (err == 0.f && fabsf(s) < P.box) return f2d(nearest_f(s, P));
-  const double d = dsub(f2d(x), f2d(q));
-  return P.periodic ? nearest_d(d, P) : d;
+  return sep_fp64_double(x, q, P.periodic, P.box, P.boxhalf);
 }
 
 __device__ __forceinline__ double walk_fp64(const Ctx &c, const Target &t, int *ninter)
 {
   const DevParams &P = c.P;
-  double pot_d = (double)__fdiv_rn(t.mself, P.eps);
-  const double th2d = (double)P.theta2;
+  double pot_d = f2d(__fdiv_rn(t.mself, P.eps));
+  const double th2d = P.theta2d;
   int n = 0;
   int cur = t.nxt;
   const int end = t.end;
@@ -303,7 +370,7 @@ __device__ __forceinline__ double walk_fp64(const Ctx &c, const Target &t, int *
       const int sk = nm.y;
       cur = (unsigned)(sk - cur - 1) < (unsigned)(end - cur - 1) ? sk : end;
       n++;
-      pot_d = dadd(pot_d, fp64_contrib(r2, (double)na.w, P));
+      pot_d = dadd(pot_d, fp64_contrib(r2, f2d(na.w), P));
     }
   }
   *ninter = n;
