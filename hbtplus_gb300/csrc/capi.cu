@@ -8,7 +8,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -37,6 +36,13 @@ struct Carver {
   }
 };
 
+// A small-subhalo call's input besides the particles, one copy: the kernel's queue
+// counters, the offsets, the states and the size order.
+static size_t call_bytes(long long S)
+{
+  return 10 * sizeof(int) + sizeof(long long) * (S + 1) + sizeof(hbtu_state) * S + sizeof(int) * S;
+}
+
 static void carve(Carver &cv, Ctx &c, Staging &sg, long long N, long long S, bool sibling)
 {
   const long long maxchunks = N / kChunk + S + 2;
@@ -62,7 +68,9 @@ static void carve(Carver &cv, Ctx &c, Staging &sg, long long N, long long S, boo
   c.plan_cnt = cv.take<int4>(S);
   c.plan_cnt2 = cv.take<int4>(S);
   c.plan_inter = cv.take<long long>(S);
-  c.small_next = cv.take<int>(1);
+  c.small_next = cv.take<int>(10);
+  c.small_list = cv.take<int>(3 * S);
+  sg.call = cv.take<char>(call_bytes(S));
   c.part_info = cv.take<int>(8 * S);
   c.seg_bbox = cv.take<unsigned>(6 * S);
   c.chunk_sums = cv.take<double>(24 * maxchunks);
@@ -190,20 +198,73 @@ hbtu_status ensure_workspace(hbtu_handle *h, long long N, long long S)
   return grow_workspace(h, workspace_bytes(N, S));
 }
 
-void init_states(const hbtu_handle *h, long long S, const int64_t *offsets, const hbtu_state *st,
-                 std::vector<SegState> &segs, std::vector<int> &segoff)
+// Subhaloes by size, largest first (equal sizes in input order).
+void order_by_size(const int64_t *offsets, long long S, long long nmax, std::vector<int> &order)
 {
-  const long long ms = h->params.max_sample_size;
-  segs.assign(S, SegState());
-  segoff.resize(S + 1);
-  for (long long s = 0; s <= S; s++) segoff[s] = (int)offsets[s];
-  for (long long s = 0; s < S; s++)
-    init_segment(segs[s], (int)offsets[s], (int)(offsets[s + 1] - offsets[s]), st[s], ms);
+  order.resize(S);
+  for (long long s = 0; s < S; s++) order[s] = (int)s;
+  std::vector<int> other(S);
+  constexpr int kBits = 11, kBins = 1 << kBits;
+  std::vector<int> at(kBins);
+  for (int shift = 0; shift < 31 && (nmax >> shift) > 0; shift += kBits) {  // LSD radix on nmax - n
+    std::fill(at.begin(), at.end(), 0);
+    auto digit = [&](int s) {
+      return (int)(((nmax - (offsets[s + 1] - offsets[s])) >> shift) & (kBins - 1));
+    };
+    for (int s : order) at[digit(s)]++;
+    int run = 0;
+    for (int &x : at) {
+      const int k = x;
+      x = run;
+      run += k;
+    }
+    for (int s : order) other[at[digit(s)]++] = s;
+    order.swap(other);
+  }
+}
+
+// A call whose subhaloes are all small enough (small.cu): its input besides the
+// particles goes to the device in one copy from a pinned buffer.
+hbtu_status stage_small_call(hbtu_handle *h, long long S, const int64_t *offsets,
+                             const hbtu_state *st, const std::vector<int> &order, Ctx &c,
+                             Staging &sg, SmallCall &io)
+{
+  const size_t bytes = call_bytes(S);
+  if (bytes > h->pin_bytes) {
+    if (h->pin) cudaFreeHost(h->pin);
+    h->pin = nullptr;
+    h->pin_bytes = 0;
+    if (cudaMallocHost(&h->pin, bytes + bytes / 4) != cudaSuccess) {
+      cudaGetLastError();
+      h->pin = nullptr;
+      return fail(h, HBTU_ERR_OUT_OF_MEMORY, "pinned staging buffer");
+    }
+    h->pin_bytes = bytes + bytes / 4;
+  }
+  int T[3];
+  small_classes(offsets, order.data(), (int)S, io.jobs, T);
+  const int queue[10] = {0, 0, 0, io.jobs[0], io.jobs[1], io.jobs[2], T[0], T[1], T[2], 0};
+  size_t o = 0;
+  auto put = [&](const void *src, size_t n) {
+    memcpy(h->pin + o, src, n);
+    char *dev = sg.call + o;
+    o += n;
+    return dev;
+  };
+  c.small_next = (int *)put(queue, sizeof(queue));
+  io.off = (const long long *)put(offsets, sizeof(long long) * (S + 1));
+  io.st = (const hbtu_state *)put(st, sizeof(hbtu_state) * S);
+  io.order = (const int *)put(order.data(), sizeof(int) * S);
+  HBTU_CUDA(cudaMemcpyAsync(sg.call, h->pin, bytes, cudaMemcpyHostToDevice, c.st));
+  return HBTU_OK;
 }
 
 // Shared set-up of a call: checks, workspace, staging, segment states, init kernel.
+// With `small`, a call whose subhaloes all fit the per-subhalo kernel is set up
+// for it instead (small->order is then not null).
 hbtu_status setup_call(hbtu_handle *h, const hbtu_particles *p, long long S, const int64_t *offsets,
-                       const hbtu_state *st, Ctx &c, Staging &sg, bool &host)
+                       const hbtu_state *st, Ctx &c, Staging &sg, bool &host,
+                       SmallCall *small = nullptr, int *nmax_out = nullptr)
 {
   if (!h || !p || !offsets || !st || S < 0)
     return fail(h, HBTU_ERR_INVALID_ARGUMENT, "null handle, particles, offsets or states");
@@ -211,9 +272,12 @@ hbtu_status setup_call(hbtu_handle *h, const hbtu_particles *p, long long S, con
     return fail(h, HBTU_ERR_INVALID_ARGUMENT, "particles.location must be HBTU_HOST or HBTU_DEVICE");
   host = p->location == HBTU_HOST;
   if (offsets[0] != 0) return fail(h, HBTU_ERR_INVALID_ARGUMENT, "offsets[0] must be 0");
-  for (long long s = 0; s < S; s++)
+  long long nmax = 0;
+  for (long long s = 0; s < S; s++) {
     if (offsets[s + 1] < offsets[s])
       return fail(h, HBTU_ERR_INVALID_ARGUMENT, "offsets must be non-decreasing");
+    nmax = std::max<long long>(nmax, offsets[s + 1] - offsets[s]);
+  }
   const long long N = offsets[S];
   if (N >= HBTU_MAX_PARTICLES)
     return fail(h, HBTU_ERR_TOO_LARGE, "more than 2^30 particles in one call");
@@ -253,17 +317,25 @@ hbtu_status setup_call(hbtu_handle *h, const hbtu_particles *p, long long S, con
   c.opt_leaf_runs = (int)h->opt_leaf_runs;
   c.opt_schedule = (int)h->opt_schedule;
   c.opt_layout = (int)h->opt_layout;
-  std::vector<SegState> segs;
-  std::vector<int> segoff, order(S);
-  init_states(h, S, offsets, st, segs, segoff);
-  for (long long s = 0; s < S; s++) order[s] = (int)s;
-  std::stable_sort(order.begin(), order.end(),
-                   [&](int a, int b) { return segs[a].n > segs[b].n; });
+  std::vector<int> order;
+  order_by_size(offsets, S, nmax, order);
   // the per-subhalo loop takes over small subhaloes (small.cu); the walk of
   // its blocks is the default one-target-per-lane schedule
   c.small_cap = h->opt_schedule == 0 ? (int)std::min<int64_t>(h->opt_small, kSmallCap) : 0;
-  c.small_per_sm = (int)h->opt_small_per_sm;
+  if (nmax_out) *nmax_out = (int)nmax;
+  if (small && S > 0 && nmax >= 2 && nmax <= c.small_cap) {
+    small->pos = pos;
+    small->vel = vel;
+    small->mass = mass;
+    return stage_small_call(h, S, offsets, st, order, c, sg, *small);
+  }
   if (S > 0) {
+    std::vector<SegState> segs(S);
+    std::vector<int> segoff(S + 1);
+    const long long ms = h->params.max_sample_size;
+    for (long long s = 0; s <= S; s++) segoff[s] = (int)offsets[s];
+    for (long long s = 0; s < S; s++)
+      init_segment(segs[s], (int)offsets[s], (int)(offsets[s + 1] - offsets[s]), st[s], ms);
     HBTU_CUDA(cudaMemcpyAsync(c.seg, segs.data(), sizeof(SegState) * S, cudaMemcpyHostToDevice,
                               c.st));
     HBTU_CUDA(cudaMemcpyAsync(c.seg_off, segoff.data(), sizeof(int) * (S + 1),
@@ -342,38 +414,7 @@ struct PhaseTimer : LoopHooks {
   }
 };
 
-hbtu_status run_loop(hbtu_handle *h, Ctx &c)
-{
-  PhaseTimer pt(h, c.st);
-  run_passes(c, max_passes_of(h->params), &pt);
-  return HBTU_OK;
-}
-
 }  // namespace
-
-void init_segment(SegState &g, int off, int n, const hbtu_state &st, long long maxsample)
-{
-  memset(&g, 0, sizeof(g));
-  g.off = off;
-  g.n = n;
-  g.status = n <= 1 ? SEG_TRIVIAL : SEG_ACTIVE;
-  g.nbound = g.nlast = n;
-  g.mode = MODE_FULL;
-  g.first_mb = INT_MAX;
-  const bool sampling = maxsample > 0 && n > maxsample;
-  g.t0 = 0;
-  g.ntree = sampling ? (int)maxsample : n;
-  g.mfac = sampling ? (float)n / (float)maxsample : 1.f;  // (HBTReal)Nlast/MaxSampleSize
-  g.ntgt = n;
-  g.tgt_mode = sampling ? 2 : 0;
-  for (int j = 0; j < 3; j++) {
-    g.ref_pos[j] = st.ref_pos[j];
-    g.ref_vel[j] = st.ref_vel[j];
-    g.mb_pos[j] = st.mostbound_pos[j];
-    g.mb_vel[j] = st.mostbound_vel[j];
-  }
-  g.mb_id = st.mostbound_id;
-}
 
 void read_plan(Ctx &c)
 {
@@ -550,6 +591,7 @@ hbtu_status hbtu_destroy(hbtu_handle *h)
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->ws) cudaFree(h->ws);
   if (h->plan_host) cudaFreeHost(h->plan_host);
+  if (h->pin) cudaFreeHost(h->pin);
   for (cudaEvent_t e : h->events) cudaEventDestroy(e);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   delete h;
@@ -660,15 +702,29 @@ hbtu_status hbtu_unbind_batch(hbtu_handle *h, const hbtu_particles *p, int64_t n
     const long long launches0 = g_launches;
     HBTU_CUDA(cudaSetDevice(h->device));
     HBTU_CUDA(cudaEventRecord(event_at(h, 0), h->stream));
-    hbtu_status rc = setup_call(h, p, nsub, offsets, st, c, sg, host);
+    SmallCall small = {};
+    int nmax = 0;
+    hbtu_status rc = setup_call(h, p, nsub, offsets, st, c, sg, host, &small, &nmax);
     if (rc != HBTU_OK) return rc;
     if (nsub == 0) return HBTU_OK;
-    run_loop(h, c);
     const long long N = c.N;
     long long *ord = host ? sg.order : (long long *)order_out;
     float *en = host ? sg.energy : energy_out;
     hbtu_result *rs = host ? sg.res : res;
-    launch_finalize(c, (int64_t *)ord, en, rs);
+    PhaseTimer pt(h, c.st);
+    if (small.order) {
+      small.order_out = (int64_t *)ord;
+      small.energy_out = en;
+      small.res = rs;
+      pt.small_begin();
+      launch_small_call(c, small, nmax, max_passes_of(h->params));
+      pt.small_end();
+      for (int64_t s = 0; s < nsub; s++)
+        h->stats.small_subhaloes += offsets[s + 1] - offsets[s] > 1;
+    } else {
+      run_passes(c, max_passes_of(h->params), &pt);
+      launch_finalize(c, (int64_t *)ord, en, rs);
+    }
     if (host) {
       if (N > 0) {
         HBTU_CUDA(cudaMemcpyAsync(order_out, ord, sizeof(long long) * N, cudaMemcpyDeviceToHost,
@@ -679,6 +735,7 @@ hbtu_status hbtu_unbind_batch(hbtu_handle *h, const hbtu_particles *p, int64_t n
     }
     HBTU_CUDA(cudaEventRecord(event_at(h, 1), c.st));
     HBTU_CUDA(cudaStreamSynchronize(c.st));
+    if (small.order) pt.collect();
     {
       float ms = 0.f;
       HBTU_CUDA(cudaEventElapsedTime(&ms, h->events[0], h->events[1]));

@@ -235,9 +235,9 @@ struct Ctx {
   double *e_part;
   // the per-subhalo loop (small.cu): it takes over once every active
   // subhalo's list holds at most small_cap particles (0: never)
-  int *small_next;   // work-queue counter
+  int *small_next;   // three work queues (large, medium, short lists): next jobs, counts, threads
+  int *small_list;   // 3 S: their jobs, S each
   int small_cap;
-  int small_per_sm;  // blocks per SM of its persistent launch
 };
 
 // launchers (tree.cu)
@@ -262,12 +262,28 @@ void launch_segment_sums(Ctx &c, const double *x, double *out);
 // (direct.cu) exact FP64 potentials of particles tidx[0..nt) from all n particles
 void direct_potential_fp64(const DevParams &P, const float4 *pm, int n, const int *tidx, int nt,
                            double *out, double *partial, int nsplit, cudaStream_t st);
-// (small.cu) the remaining passes of every active subhalo, one block per
-// subhalo; `cap` bounds their energy lists (at most kSmallCap particles)
+// (small.cu) the remaining passes of every active subhalo, one block or warp
+// per subhalo; `cap` bounds their energy lists (at most kSmallCap particles)
 constexpr int kSmallCap = 2048;
 constexpr int kSmallDefault = 2048;
 void launch_small(Ctx &c, int cap, int nactive, int max_passes);
-size_t small_smem_bytes(int cap);
+// A whole call whose subhaloes all hold at most kSmallCap particles, in the
+// same kernel: set-up, every pass and the results.
+struct SmallCall {
+  const float *pos, *vel, *mass;
+  const hbtu_state *st;    // per subhalo
+  const long long *off;    // S + 1
+  const int *order;        // subhaloes by size, largest first
+  int jobs[3];             // lists of each size class (small_classes)
+  int64_t *order_out;
+  float *energy_out;
+  hbtu_result *res;
+};
+constexpr int kSmallWarpCap = 128;    // lists up to this long: one warp each
+constexpr int kSmallMediumCap = 512;  // lists up to this long: four warps, longer ones a block
+// The lists of each size class and the threads of its groups.
+void small_classes(const int64_t *offsets, const int *order, int S, int (&n)[3], int (&T)[3]);
+void launch_small_call(Ctx &c, const SmallCall &io, int cap, int max_passes);
 // launchers (loop.cu)
 void launch_init(Ctx &c, const float *pos, const float *vel, const float *mass,
                  const long long *id);

@@ -16,6 +16,7 @@ struct Staging {
   hbtu_result *res;
   float *grad;   // 7 per particle: host-located gradient staging
   double *esum;  // per subhalo
+  char *call;    // a small-subhalo call's input besides the particles
 };
 
 // Bytes of device workspace for N particles in S subhaloes, and the carving of
@@ -24,9 +25,6 @@ struct Staging {
 size_t workspace_bytes(long long N, long long S, bool sibling = true);
 void carve_workspace(char *base, Ctx &c, Staging &sg, long long N, long long S,
                      bool sibling = true);
-
-// Loop state of subhalo s before its first pass.
-void init_segment(SegState &g, int off, int n, const hbtu_state &st, long long maxsample);
 
 // Optional tracing of the loop: per-phase marks and counters.
 struct LoopHooks {

@@ -16,6 +16,8 @@ struct hbtu_handle {
   char *ws = nullptr;
   size_t ws_bytes = 0;
   hbtu::PassPlan *plan_host = nullptr;
+  char *pin = nullptr;  // pinned staging of a call's offsets, states and order
+  size_t pin_bytes = 0;
   // tracing
   hbtu_stats stats{};
   bool timing = false;

@@ -21,6 +21,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <string>
 
@@ -85,6 +86,33 @@ struct SegState {
   float e0;  // Elist[0].E at disruption
   long long evals, interactions;
 };
+
+// Loop state of a subhalo before its first pass (host: the batch path's states;
+// device: small.cu's).
+__host__ __device__ inline void init_segment(SegState &g, int off, int n, const hbtu_state &st,
+                                             long long maxsample)
+{
+  memset(&g, 0, sizeof(g));
+  g.off = off;
+  g.n = n;
+  g.status = n <= 1 ? SEG_TRIVIAL : SEG_ACTIVE;
+  g.nbound = g.nlast = n;
+  g.mode = MODE_FULL;
+  g.first_mb = 0x7fffffff;
+  const bool sampling = maxsample > 0 && n > maxsample;
+  g.t0 = 0;
+  g.ntree = sampling ? (int)maxsample : n;
+  g.mfac = sampling ? (float)n / (float)maxsample : 1.f;  // (HBTReal)Nlast/MaxSampleSize
+  g.ntgt = n;
+  g.tgt_mode = sampling ? 2 : 0;
+  for (int j = 0; j < 3; j++) {
+    g.ref_pos[j] = st.ref_pos[j];
+    g.ref_vel[j] = st.ref_vel[j];
+    g.mb_pos[j] = st.mostbound_pos[j];
+    g.mb_vel[j] = st.mostbound_vel[j];
+  }
+  g.mb_id = st.mostbound_id;
+}
 
 // Totals the host reads once per pass.
 struct PassPlan {

@@ -209,15 +209,17 @@ hbtu_status hbtu_get_stats(const hbtu_handle *h, hbtu_stats *out);
 hbtu_status hbtu_reset_stats(hbtu_handle *h);
 
 /* Tuning options of a handle (results do not depend on them):
- *   "small_cutoff"    (default 2048, at most 2048; 0: off) from the first
- *                     round of the loop at which every active subhalo's
- *                     energy list holds at most this many particles, one
- *                     persistent launch finishes them all, one thread block
- *                     per subhalo running its remaining passes (a work queue
- *                     in size order); before it, every active subhalo
- *                     advances one pass per round of batch kernels.  With
+ *   "small_cutoff"    (default 2048, at most 2048; 0: off) a call whose
+ *                     subhaloes all hold at most this many particles runs in
+ *                     one persistent launch, one to several warps (or blocks)
+ *                     per subhalo, passes and results included; in a larger
+ *                     call that launch finishes the passes from the first
+ *                     round at which every active subhalo's energy list is
+ *                     that short (before it, every active subhalo advances
+ *                     one pass per round of batch kernels).  With
  *                     walk_schedule 1 it is off.
- *   "small_blocks_per_sm" (default 1, 1..8) blocks per SM of that launch.
+ *   "small_blocks_per_sm" (default 1, 1..8) accepted and kept; the launch now
+ *                     takes as many blocks as its lists need and the chip holds.
  *   "walk_schedule"   how the FP32 walk visits nodes: 0 (default) every
  *                     lane walks its own target; 1 a warp visits the smallest
  *                     node index any of its targets waits at (broadcast loads).
