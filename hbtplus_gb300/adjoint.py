@@ -22,15 +22,11 @@ import numpy as np
 import torch
 
 from . import _lib
-from .unbind import Unbinder, _state
+from .unbind import Unbinder, state_array
 
 
 def _states(ref_pos, ref_vel):
-    nsub = len(ref_pos)
-    sts = (_lib.hbtu_state * max(nsub, 1))()
-    for s in range(nsub):
-        sts[s] = _state(ref_pos[s], ref_vel[s], ref_pos[s], ref_vel[s], -1)
-    return sts
+    return state_array(ref_pos, ref_vel, ref_pos, ref_vel, np.full(len(ref_pos), -1, np.int64))
 
 
 def bound_subset(batch: dict, order, results) -> dict:

@@ -261,10 +261,11 @@ hbtu_status stage_small_call(hbtu_handle *h, long long S, const int64_t *offsets
 
 // Shared set-up of a call: checks, workspace, staging, segment states, init kernel.
 // With `small`, a call whose subhaloes all fit the per-subhalo kernel is set up
-// for it instead (small->order is then not null).
+// for it instead (small->order is then not null).  one_pass: a single full pass
+// over every particle follows: no sampling, lists of one particle take part.
 hbtu_status setup_call(hbtu_handle *h, const hbtu_particles *p, long long S, const int64_t *offsets,
                        const hbtu_state *st, Ctx &c, Staging &sg, bool &host,
-                       SmallCall *small = nullptr, int *nmax_out = nullptr)
+                       SmallCall *small = nullptr, int *nmax_out = nullptr, bool one_pass = false)
 {
   if (!h || !p || !offsets || !st || S < 0)
     return fail(h, HBTU_ERR_INVALID_ARGUMENT, "null handle, particles, offsets or states");
@@ -332,10 +333,12 @@ hbtu_status setup_call(hbtu_handle *h, const hbtu_particles *p, long long S, con
   if (S > 0) {
     std::vector<SegState> segs(S);
     std::vector<int> segoff(S + 1);
-    const long long ms = h->params.max_sample_size;
+    const long long ms = one_pass ? 0 : h->params.max_sample_size;
     for (long long s = 0; s <= S; s++) segoff[s] = (int)offsets[s];
-    for (long long s = 0; s < S; s++)
+    for (long long s = 0; s < S; s++) {
       init_segment(segs[s], (int)offsets[s], (int)(offsets[s + 1] - offsets[s]), st[s], ms);
+      if (one_pass && segs[s].n == 1) segs[s].status = SEG_ACTIVE;
+    }
     HBTU_CUDA(cudaMemcpyAsync(c.seg, segs.data(), sizeof(SegState) * S, cudaMemcpyHostToDevice,
                               c.st));
     HBTU_CUDA(cudaMemcpyAsync(c.seg_off, segoff.data(), sizeof(int) * (S + 1),
@@ -782,26 +785,13 @@ hbtu_status hbtu_energy_gradient(hbtu_handle *h, const hbtu_particles *p, int64_
     Staging sg;
     bool host = true;
     const long long launches0 = g_launches;
-    // a single full pass over every particle: no sampling
-    const int64_t saved = h->params.max_sample_size;
-    h->params.max_sample_size = 0;
-    hbtu_status rc = setup_call(h, p, nsub, offsets, st, c, sg, host);
-    h->params.max_sample_size = saved;
+    hbtu_status rc = setup_call(h, p, nsub, offsets, st, c, sg, host, nullptr, nullptr, true);
     if (rc != HBTU_OK) return rc;
     if (nsub == 0) return HBTU_OK;
     const long long N = c.N;
     c.grad_pos = grad_pos ? (host ? sg.grad : grad_pos) : nullptr;
     c.grad_vel = grad_vel ? (host ? sg.grad + 3 * N : grad_vel) : nullptr;
     c.grad_mass = grad_mass ? (host ? sg.grad + 6 * N : grad_mass) : nullptr;
-    // every subhalo with at least one particle takes part (n == 1 included)
-    std::vector<SegState> segs(nsub);
-    HBTU_CUDA(cudaMemcpyAsync(segs.data(), c.seg, sizeof(SegState) * nsub, cudaMemcpyDeviceToHost,
-                              c.st));
-    HBTU_CUDA(cudaStreamSynchronize(c.st));
-    for (auto &g : segs)
-      if (g.n >= 1) g.status = SEG_ACTIVE;
-    HBTU_CUDA(cudaMemcpyAsync(c.seg, segs.data(), sizeof(SegState) * nsub, cudaMemcpyHostToDevice,
-                              c.st));
     if (N > 0) HBTU_CUDA(cudaMemsetAsync(c.e_part, 0, sizeof(double) * N, c.st));
     launch_plan(c, 0);
     launch_bbox_cube(c, c.N / kChunk + c.S + 1);
@@ -903,18 +893,9 @@ hbtu_status hbtu_binding_energies(hbtu_handle *h, const hbtu_particles *p, int64
     Ctx c;
     Staging sg;
     bool host = true;
-    // one exact full pass: no sampling
-    const int64_t saved = h->params.max_sample_size;
-    h->params.max_sample_size = 0;
-    hbtu_status rc = setup_call(h, p, 1, offsets, &st, c, sg, host);
-    h->params.max_sample_size = saved;
+    hbtu_status rc = setup_call(h, p, 1, offsets, &st, c, sg, host, nullptr, nullptr, true);
     if (rc != HBTU_OK) return rc;
     if (n == 0) return HBTU_OK;
-    SegState one;
-    HBTU_CUDA(cudaMemcpyAsync(&one, c.seg, sizeof(SegState), cudaMemcpyDeviceToHost, c.st));
-    HBTU_CUDA(cudaStreamSynchronize(c.st));
-    one.status = SEG_ACTIVE;  // n == 1 runs the pass too
-    HBTU_CUDA(cudaMemcpyAsync(c.seg, &one, sizeof(SegState), cudaMemcpyHostToDevice, c.st));
     c.pot_out = (host || !potential_out) ? sg.pot : potential_out;
     launch_plan(c, 0);
     launch_bbox_cube(c, c.N / kChunk + 2);

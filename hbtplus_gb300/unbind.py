@@ -181,6 +181,25 @@ def _state(ref_pos, ref_vel, mb_pos, mb_vel, mb_id) -> _lib.hbtu_state:
     return s
 
 
+def _host(values) -> np.ndarray:
+    """values (an array, a sequence or a tensor on any device) as a numpy array."""
+    return values.detach().cpu().numpy() if hasattr(values, "detach") else np.asarray(values)
+
+
+def state_array(ref_pos, ref_vel, mostbound_pos, mostbound_vel, mostbound_id) -> C.Array:
+    """A ctypes array of hbtu_state, one per subhalo, from arrays of its fields."""
+    nsub = len(mostbound_id)
+    sts = (_lib.hbtu_state * max(nsub, 1))()
+    rec = np.frombuffer(sts, dtype=np.dtype(_lib.hbtu_state), count=nsub)
+    for name, values in (("ref_pos", ref_pos), ("ref_vel", ref_vel),
+                         ("mostbound_pos", mostbound_pos), ("mostbound_vel", mostbound_vel),
+                         ("mostbound_id", mostbound_id)):
+        if nsub:
+            v = _host(values)
+            rec[name] = v[:nsub, :3] if v.ndim > 1 else v[:nsub]
+    return sts
+
+
 def _ptr(a: np.ndarray) -> int:
     return a.ctypes.data if a is not None and a.size else 0
 
@@ -273,13 +292,7 @@ class Unbinder:
         nsub = len(off) - 1
         ntot = int(off[-1])
         p, keep = self._host_particles(batch)
-        sts = (_lib.hbtu_state * max(nsub, 1))()
-        for s in range(nsub):
-            o = int(off[s])
-            mb_id = batch["mostbound_id"][s] if "mostbound_id" in batch else (
-                batch["id"][o] if off[s + 1] > o else -1)
-            sts[s] = _state(batch["ref_pos"][s], batch["ref_vel"][s], batch["mostbound_pos"][s],
-                            batch["mostbound_vel"][s], mb_id)
+        sts = self.make_states(batch)
         order = np.zeros(max(ntot, 1), np.int64)
         energy = np.zeros(max(ntot, 1), np.float32)
         res = (_lib.hbtu_result * max(nsub, 1))()
@@ -421,16 +434,17 @@ class Unbinder:
 
     @staticmethod
     def make_states(batch: dict):
-        off = batch["offsets"]
+        off = np.asarray(_host(batch["offsets"]), np.int64)
         nsub = len(off) - 1
-        sts = (_lib.hbtu_state * max(nsub, 1))()
-        for s in range(nsub):
-            o = int(off[s])
-            mb_id = batch["mostbound_id"][s] if "mostbound_id" in batch else (
-                batch["id"][o] if off[s + 1] > o else -1)
-            sts[s] = _state(batch["ref_pos"][s], batch["ref_vel"][s], batch["mostbound_pos"][s],
-                            batch["mostbound_vel"][s], mb_id)
-        return sts
+        if "mostbound_id" in batch:
+            mb_id = _host(batch["mostbound_id"])[:nsub]
+        else:  # each list's first particle
+            ids = _host(batch["id"])
+            mb_id = np.full(nsub, -1, np.int64)
+            some = off[1:] > off[:-1]
+            mb_id[some] = ids[off[:-1][some]]
+        return state_array(batch["ref_pos"], batch["ref_vel"], batch["mostbound_pos"],
+                           batch["mostbound_vel"], mb_id)
 
 
 def results_from_bytes(buf: bytes, nsub: int):
