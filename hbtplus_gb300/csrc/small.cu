@@ -396,10 +396,12 @@ __device__ void walk_targets(const Group &g, const Ctx &c, int s, int P0, const 
   const int tm = sg.tgt_mode;
   const int count = tm == 1 ? sg.coh_n : sg.ntgt;
   int total = 0;
-  for (int w = first; w < count; w += step) {
-    int epos, pid;
-    bool active = true;
-    if (tm == 0) {  // full pass: tree leaves in Morton order
+  const int lane = threadIdx.x & 31;
+  for (int w = first; w - lane < count; w += step) {  // whole warps
+    int epos = 0, pid = 0;
+    bool active = w < count;
+    if (!active) {
+    } else if (tm == 0) {  // full pass: tree leaves in Morton order
       epos = sval[w];
       pid = c.epid[epos];
       c.coh_pid[P0 + w] = pid;
