@@ -246,15 +246,28 @@ void launch_tree_build(Ctx &c, const PassPlan &pl);
 // launchers (walk.cu)
 void launch_walk(Ctx &c, const PassPlan &pl);
 void launch_sibling_layout(Ctx &c, const PassPlan &pl);
+// The FP32 lane walk of two neighbouring targets per lane (walk_pair): from
+// kPairMin targets on, 5 warps of pairs per scheduler.  Fewer lanes than that leave
+// the chip waiting on each walk's chain of loads (first pass of a subhalo of 1.1e5
+// particles: 937 us in pairs, 623 one by one; 1.6e5: 1014 and 967; 2.2e5: 1174 and
+// 1228; 3.4e5: 1607 and 2278; 1.1e6: 4.5 and 5.5 ms; 2.7e7: 122 and 160 ms).
+// Targets in list order are no neighbours: 780,000 of them took 810 us against 765.
+// The gradient's walk stays with one target per lane.
+constexpr int kPairMin = 152 * 4 * 5 * 64;
+inline bool pair_walk(const Ctx &c, const PassPlan &pl)
+{
+  return c.P.precision != HBTU_PRECISION_FP64 && c.opt_schedule == 0 && pl.nlist == 0 &&
+         pl.ntgt_total >= kPairMin && !(c.grad_pos || c.grad_vel || c.grad_mass);
+}
 // The FP32 lane walk over the sibling-block records (the tree build then makes
 // them): for trees of at least kSiblingMinTree particles in all, where the
 // faster walk pays for the extra pass over the nodes (the small trees of
-// correction passes do not).
+// correction passes do not), unless walk_pair takes the pass.
 constexpr int kSiblingMinTree = 1 << 16;
 inline bool sibling_walk(const Ctx &c, const PassPlan &pl)
 {
   return c.P.precision != HBTU_PRECISION_FP64 && c.opt_schedule == 0 && c.opt_layout && c.nd2 &&
-         pl.ntree_total >= kSiblingMinTree;
+         pl.ntree_total >= kSiblingMinTree && !pair_walk(c, pl);
 }
 void launch_grad_walk(Ctx &c, const PassPlan &pl);
 // per-subhalo sums of a per-particle double array (input positions), deterministic

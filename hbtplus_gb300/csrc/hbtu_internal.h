@@ -123,6 +123,7 @@ struct PassPlan {
   int nsort_total;  // elements of the unbound-part sort
   int nchunks_bound;
   int nrefine;
+  int norder, nlist;     // subhaloes whose targets follow an earlier pass's order, the list
   int error;             // a sort's look-back wait ran out
   int max_nlast;         // longest energy list of an active subhalo
   long long inter_done;  // walk interactions summed so far, all subhaloes
@@ -165,11 +166,11 @@ struct CudaError {
 
 bool launch_overlap();  // false when HBTU_LAUNCH_OVERLAP=0 (read once)
 
-// kernel<<<grid, block, smem, st>>>(args...) with programmatic stream
-// serialisation; only for kernels that open with HBTU_KERNEL_PROLOGUE.
+// kernel<<<grid, block, smem, st>>>(args...), with programmatic stream
+// serialisation if `ahead`.
 template <typename... P, typename... A>
-inline void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                     A... args)
+inline void launch_attr(bool ahead, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                        cudaStream_t st, A... args)
 {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -180,10 +181,25 @@ inline void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, c
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = at;
-  cfg.numAttrs = launch_overlap() ? 1 : 0;
+  cfg.numAttrs = ahead ? 1 : 0;
   HBTU_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
+// Only for kernels that open with HBTU_KERNEL_PROLOGUE.
+template <typename... P, typename... A>
+inline void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                     A... args)
+{
+  launch_attr(launch_overlap(), kernel, grid, block, smem, st, args...);
+}
+
+// After all of the kernel before it.
+template <typename... P, typename... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t st, A... args)
+{
+  launch_attr(false, kernel, grid, block, smem, st, args...);
+}
 
 // ---------------- primitives (prims.cu) ----------------
 // Exclusive scan of n int64 values (in may equal out).  tmp: scan_tmp_bytes(n).

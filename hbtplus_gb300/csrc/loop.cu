@@ -191,7 +191,7 @@ __device__ int get_pass(const Ctx &c, int s, int *v)
   const bool act = sg.status == SEG_ACTIVE;
   v[0] = act ? sg.ntree : 0;
   v[1] = act ? (sg.ntree + kChunk - 1) / kChunk : 0;
-  v[2] = act ? (sg.tgt_mode == 1 ? sg.coh_n : sg.ntgt) : 0;
+  v[2] = act && sg.tgt_mode == 2;  // summed only
   v[3] = sg.ub_hi - sg.ub_lo;
   return 0;
 }
@@ -200,8 +200,9 @@ __device__ int get_targets_sorted(const Ctx &c, int k, int *v)
 {
   const SegState &sg = c.seg[c.seg_order[k]];
   const bool act = sg.status == SEG_ACTIVE;
-  v[0] = act ? (sg.tgt_mode == 1 ? sg.coh_n : sg.ntgt) : 0;
-  v[1] = v[2] = v[3] = 0;
+  v[0] = act ? sg.ntgt : 0;
+  v[1] = v[2] = 0;
+  v[3] = act && sg.tgt_mode == 1;  // summed only
   return 0;
 }
 __device__ int get_bound(const Ctx &c, int s, int *v)
@@ -333,6 +334,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(Ctx c, int mode, int gath
     if (threadIdx.x == 0) {
       c.plan->ntree_total = tot[0];
       c.plan->nchunks_tree = tot[1];
+      c.plan->nlist = tot[2];
       c.plan->nsort_total = tot[3];
       c.plan->max_levels = 0;
     }
@@ -342,12 +344,14 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(Ctx c, int mode, int gath
       if (threadIdx.x == 0) {
         c.plan->ntgt_total = tot[0];
         c.plan->nactive = tot[1];
+        c.plan->norder = tot[3];
       }
     } else {
       plan_scan4_thread<get_targets_sorted>(c.S, c, c.tgt_base, nullptr, nullptr, nullptr, tot);
       if (threadIdx.x == 0) {
         c.plan->ntgt_total = tot[0];
         c.plan->nactive = nact;
+        c.plan->norder = tot[3];
       }
     }
   } else if (mode == 1) {

@@ -16,9 +16,9 @@
 // the reference takes them; the potential is summed in float with
 // compensation and formed in double once per target (no double arithmetic in
 // the loop: this GPU's FP64 rate is 1/64 of its FP32 rate).  Two schedules:
-//   lane (default): every lane walks its own target, one 32-byte node record
-//     per step; large blocks keep a block's neighbouring targets on one SM,
-//     so the walks share L1;
+//   lane (default): every lane walks its own target, or in large launches two
+//     neighbouring ones at once, one 32-byte node record per step; large blocks
+//     keep a block's neighbouring targets on one SM, so the walks share L1;
 //   warp: the warp visits the smallest index any of its targets waits at, so
 //     each node is a broadcast load (kept as an option for comparison).
 // FP64: absolute float coordinates, NEAREST per interaction, every operation
@@ -59,15 +59,84 @@ __device__ __forceinline__ void load_target(const Ctx &c, int w, int total, Targ
     c.coh_pid[sg.off + local] = pid;
     active = true;
   } else if (tm == 1) {  // correction pass: last full pass's Morton order, still bound
-    pid = c.coh_pid[sg.off + local];
+    pid = c.epid2[sg.off + local];  // launch_bound_order
     epos = c.epos_of_pid[pid];
-    active = (epos - sg.off) < sg.ntgt;
+    c.coh_pid[sg.off + local] = pid;
+    active = true;
   } else {  // list order
     epos = sg.off + local;
     pid = c.epid[epos];
     active = true;
   }
   init_target<kRel>(c, sg, s, epos, pid, active, 2 * c.tree_base[s], t);
+}
+
+// Correction passes walk the particles still bound, in the Morton order of the
+// last full pass.  That pass's list is first rid of the particles removed since,
+// which left lanes idle and kept the neighbours of a pair apart (correction pass
+// of a 2.7e7-particle host: 94 ms with the removed ones in the list, one target
+// per lane; 93 without them, 92 in pairs with them, 65 in pairs without).  The new
+// list goes to epid2, free between the tree build and the partition; the walk
+// copies it to coh_pid (load_target).  Bandwidth- and gather-bound: 56 us for the
+// 1.3e6 particles of a tracking step.
+// k_order_count leaves per 32 list positions x the bits of the still bound and y
+// how many come before them in the block, and per block their count (scanned next).
+constexpr int kOrderBlock = 1024;
+
+__global__ void __launch_bounds__(kOrderBlock) k_order_count(Ctx c)
+{
+  HBTU_KERNEL_PROLOGUE();
+  __shared__ int wsum[32];
+  const int p = blockIdx.x * kOrderBlock + threadIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  bool keep = false;
+  if (p < c.N) {
+    const SegState &sg = c.seg[c.pseg[p]];
+    keep = sg.status == SEG_ACTIVE && sg.tgt_mode == 1 && p - sg.off < sg.coh_n &&
+           c.epos_of_pid[c.coh_pid[p]] - sg.off < sg.ntgt;
+  }
+  const unsigned bits = __ballot_sync(0xffffffffu, keep);
+  if (lane == 0) wsum[w] = __popc(bits);
+  __syncthreads();
+  if (w == 0) {
+    const int own = wsum[lane];
+    int x = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    wsum[lane] = x - own;
+    if (lane == 31) c.pX[blockIdx.x] = x;
+  }
+  __syncthreads();
+  if (lane == 0) reinterpret_cast<uint2 *>(c.pcode)[p >> 5] = make_uint2(bits, wsum[w]);
+}
+
+__global__ void __launch_bounds__(kWB) k_order_write(Ctx c)
+{
+  HBTU_KERNEL_PROLOGUE();
+  const int p = blockIdx.x * kWB + threadIdx.x;
+  if (p >= c.N) return;
+  const uint2 *words = reinterpret_cast<const uint2 *>(c.pcode);
+  SegState &sg = c.seg[c.pseg[p]];
+  const uint2 x = words[p >> 5];
+  if (p == sg.off && sg.status == SEG_ACTIVE && sg.tgt_mode == 1) sg.coh_n = sg.ntgt;
+  if (!(x.x >> (p & 31) & 1u)) return;
+  const int o = sg.off;
+  const uint2 y = words[o >> 5];
+  const int at = (int)c.pX[p / kOrderBlock] + x.y + __popc(x.x & ((1u << (p & 31)) - 1u));
+  const int at0 = (int)c.pX[o / kOrderBlock] + y.y + __popc(y.x & ((1u << (o & 31)) - 1u));
+  c.epid2[o + at - at0] = c.coh_pid[p];
+}
+
+void launch_bound_order(Ctx &c)
+{
+  const int nb = (c.N + kOrderBlock - 1) / kOrderBlock;
+  launch_k(k_order_count, nb, kOrderBlock, 0, c.st, c);
+  HBTU_LAUNCHED();
+  exclusive_scan_i64(c.pX, c.pX, nb, c.scan_tmp, c.st);
+  launch_k(k_order_write, (c.N + kWB - 1) / kWB, kWB, 0, c.st, c);
+  HBTU_LAUNCHED();
 }
 
 // FP32 walk, warp schedule.  Leaf runs: when targets open a cell
@@ -171,15 +240,40 @@ __global__ void __launch_bounds__(kB) k_walk_fp32_lean(Ctx c, int total)
   count_interactions(c, t.s, ninter);
 }
 
+// Two neighbouring targets per lane (walk_pair).
+constexpr int kPB = 256;
+inline unsigned pair_blocks(int n) { return ((unsigned)n + 2 * kPB - 1) / (2 * kPB); }
+
+__global__ void __launch_bounds__(kPB, 4) k_walk_fp32_pair(Ctx c, int total)
+{
+  HBTU_KERNEL_PROLOGUE();
+  Target t[2];
+  const int w = 2 * (blockIdx.x * kPB + threadIdx.x);
+  load_target<true>(c, w, total, t[0]);
+  load_target<true>(c, w + 1, total, t[1]);
+  int ninter[2];
+  double pot[2];
+  walk_pair(c.nd, t, c.P, ninter, pot);
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    finish_target(c, c.seg[t[k].s], t[k], pot[k]);
+    count_interactions(c, t[k].s, ninter[k]);
+  }
+}
+
+// The walks are launched after all of the kernel before them: blocks
+// placed while its blocks still hold their SMs gather on the other SMs, and a walk
+// of few blocks never evens that out (1e5 targets after 108 blocks of 1024 threads:
+// 574 us, not 287; the unbinding of 1.1e5 particles 1.81 ms, 1.90 launched ahead).
 template <bool kSib>
 void launch_lean(Ctx &c, int n)
 {
   if (n >= 152 * 4 * 512)  // blocks of neighbouring targets share an SM's L1
-    launch_k(k_walk_fp32_lean<512, kSib, false>, (n + 511) / 512, 512, 0, c.st, c, n);
+    launch_after(k_walk_fp32_lean<512, kSib, false>, (n + 511) / 512, 512, 0, c.st, c, n);
   else if (n >= 152 * 4 * 256)
-    launch_k(k_walk_fp32_lean<256, kSib, true>, (n + 255) / 256, 256, 0, c.st, c, n);
+    launch_after(k_walk_fp32_lean<256, kSib, true>, (n + 255) / 256, 256, 0, c.st, c, n);
   else
-    launch_k(k_walk_fp32_lean<128, kSib, true>, (n + 127) / 128, 128, 0, c.st, c, n);
+    launch_after(k_walk_fp32_lean<128, kSib, true>, (n + 127) / 128, 128, 0, c.st, c, n);
 }
 
 // FP64: the reference's arithmetic, operation by operation (walk_fp64), one
@@ -292,16 +386,13 @@ __device__ __forceinline__ double walk_grad(const WNode *nodes, const Target &t,
   return dadd(dadd(base, (double)hi), -(double)comp);
 }
 
-template <int kB, bool kSib, bool kGrad>
-__global__ void __launch_bounds__(kB) k_grad_walk(Ctx c, int total)
+// The target's gradient and its term of the total energy.
+template <bool kGrad>
+__device__ __forceinline__ void finish_grad(const Ctx &c, const Target &t, double pot_sum,
+                                            const double (&acc)[3])
 {
-  HBTU_KERNEL_PROLOGUE();
-  const DevParams &P = c.P;
-  Target t;
-  load_target<true>(c, blockIdx.x * kB + threadIdx.x, total, t);
-  double acc[3];
-  const double pot_sum = walk_grad<kSib, kGrad>(kSib ? c.nd2 : c.nd, t, P, acc);
   if (!t.active) return;
+  const DevParams &P = c.P;
   const SegState &sg = c.seg[t.s];
   const double ga = ddiv((double)P.G, (double)P.a);
   const double pot = dmul(pot_sum, ga);
@@ -323,6 +414,33 @@ __global__ void __launch_bounds__(kB) k_grad_walk(Ctx c, int total)
   c.e_part[i] = 0.5 * m * k2 + 0.5 * m * pot;
 }
 
+template <int kB, bool kSib, bool kGrad>
+__global__ void __launch_bounds__(kB) k_grad_walk(Ctx c, int total)
+{
+  HBTU_KERNEL_PROLOGUE();
+  Target t;
+  load_target<true>(c, blockIdx.x * kB + threadIdx.x, total, t);
+  double acc[3];
+  const double pot = walk_grad<kSib, kGrad>(kSib ? c.nd2 : c.nd, t, c.P, acc);
+  finish_grad<kGrad>(c, t, pot, acc);
+}
+
+// The energies alone, two neighbouring targets per lane (walk_pair).
+__global__ void __launch_bounds__(kPB, 4) k_grad_walk_pair(Ctx c, int total)
+{
+  HBTU_KERNEL_PROLOGUE();
+  Target t[2];
+  const int w = 2 * (blockIdx.x * kPB + threadIdx.x);
+  load_target<true>(c, w, total, t[0]);
+  load_target<true>(c, w + 1, total, t[1]);
+  int ninter[2];
+  double pot[2];
+  const double acc[3] = {0., 0., 0.};
+  walk_pair(c.nd, t, c.P, ninter, pot);
+#pragma unroll
+  for (int k = 0; k < 2; k++) finish_grad<false>(c, t[k], pot[k], acc);
+}
+
 template <bool kSib, bool kGrad>
 void launch_grad(Ctx &c, int n)
 {
@@ -340,6 +458,7 @@ void launch_walk(Ctx &c, const PassPlan &pl)
 {
   const int n = pl.ntgt_total;
   if (n <= 0) return;
+  if (pl.norder > 0) launch_bound_order(c);
   const unsigned blocks = (n + kWB - 1) / kWB;
   if (c.P.precision == HBTU_PRECISION_FP64)
     launch_k(k_walk_fp64, blocks, kWB, 0, c.st, c, n);
@@ -347,6 +466,8 @@ void launch_walk(Ctx &c, const PassPlan &pl)
     launch_k(k_walk_fp32<true>, blocks, kWB, 0, c.st, c, n);
   else if (c.opt_schedule == 1)
     launch_k(k_walk_fp32<false>, blocks, kWB, 0, c.st, c, n);
+  else if (pair_walk(c, pl))
+    launch_after(k_walk_fp32_pair, pair_blocks(n), kPB, 0, c.st, c, n);
   else if (sibling_walk(c, pl))  // the tree build made the sibling-block records
     launch_lean<true>(c, n);
   else
@@ -360,7 +481,9 @@ void launch_grad_walk(Ctx &c, const PassPlan &pl)
   if (n <= 0) return;
   const bool grad = c.grad_pos || c.grad_vel || c.grad_mass;
   const bool sib = sibling_walk(c, pl);  // the tree build made the sibling-block records
-  if (sib && grad)
+  if (pair_walk(c, pl))  // no gradient asked for
+    launch_k(k_grad_walk_pair, pair_blocks(n), kPB, 0, c.st, c, n);
+  else if (sib && grad)
     launch_grad<true, true>(c, n);
   else if (sib)
     launch_grad<true, false>(c, n);

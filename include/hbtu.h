@@ -228,7 +228,9 @@ hbtu_status hbtu_reset_stats(hbtu_handle *h);
  *   "walk_layout"     1 (default) or 0: with walk_schedule 0, passes whose
  *                     trees hold at least 2^16 particles in all walk a copy
  *                     of the node records with every cell's children in
- *                     consecutive slots (0: the preorder records). */
+ *                     consecutive slots (0: the preorder records).  Passes of
+ *                     194560 targets and more, subhaloes with sampled
+ *                     potentials apart, always walk the preorder records. */
 hbtu_status hbtu_set_option(hbtu_handle *h, const char *name, int64_t value);
 hbtu_status hbtu_get_option(const hbtu_handle *h, const char *name, int64_t *value);
 
