@@ -317,6 +317,8 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
   s = t;
 }
 
+// As in walk_lean the next node's load is issued before the node's terms are
+// computed (1e6 targets: 5.74 -> 5.60 ms; 2000 subhaloes, 6e5 targets: 1.73 -> 1.64).
 template <bool kSib, bool kGrad>
 __device__ __forceinline__ double walk_grad(const WNode *nodes, const Target &t,
                                             const DevParams &P, double (&acc)[3])
@@ -328,56 +330,56 @@ __device__ __forceinline__ double walk_grad(const WNode *nodes, const Target &t,
   // loop, where the lanes of a warp drift apart and a double instruction would
   // issue once per drifting group of lanes
   float ax = 0.f, ay = 0.f, az = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-  int iters = 0;
-  int cur = t.nxt;
-  const int end = t.end;
-  const int steps = kSib ? max(end - t.nxt, 0) : 0;
-  while (cur < end) {
+  const int root = t.nxt;
+  const unsigned nn = t.end > root ? (unsigned)(t.end - root) : 0u;
+  if (nn > 0u) {
+    unsigned left = nn;  // steps left
+    int cur = root;
     float4 na;
     int4 nm;
     load_node(nodes, cur, na, nm);
-    const float dx = na.x - t.q[0], dy = na.y - t.q[1], dz = na.z - t.q[2];
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float lo = __int_as_float(nm.z);
-    const float up = kSib ? lo * kBandRatio : __int_as_float(nm.w);
-    bool open = r2 < lo;
-    if (r2 >= lo && r2 <= up)
-      open = exact_open(na, t.q[0], t.q[1], t.q[2], __int_as_float(nm.x & 0x7fffffff), th2d);
-    const float rinv = rsqrtf(fmaxf(r2, 1e-30f));
-    const float mass = fabsf(na.w);  // cells carry their mass with the sign bit set
-    float contrib = -mass * rinv;
-    if (r2 < h2f) contrib = softened_fp32(mass, r2, rinv, hf, hinvf);
-    contrib = open ? 0.f : contrib;
-    const float y = __fsub_rn(contrib, comp);
-    const float sum = __fadd_rn(hi, y);
-    comp = __fsub_rn(__fsub_rn(sum, hi), y);
-    hi = sum;
-    if (kGrad && !open) {
-      float w;  // gradient weight: grad phi -= m * w * dx
-      if (r2 >= h2f) {
-        w = rinv * rinv * rinv;
-      } else {
-        const float u = r2 * rinv * hinvf;
-        const float iu = hf * rinv;  // 1/u
-        const float dwp = u < 0.5f
-                              ? u * (10.666666666667f + u * u * (32.0f * u - 38.4f))
-                              : -0.066666666667f * iu * iu +
-                                    u * (21.333333333333f +
-                                         u * (-48.0f + u * (38.4f - 10.666666666667f * u)));
-        w = r2 > 0.f ? hinvf * hinvf * dwp * rinv : 0.f;
+    bool go;
+    do {
+      const float dx = na.x - t.q[0], dy = na.y - t.q[1], dz = na.z - t.q[2];
+      const float r2 = dist2(na, t.q);
+      const float lo = __int_as_float(nm.z);
+      const float up = kSib ? lo * kBandRatio : __int_as_float(nm.w);
+      bool open = r2 < lo;
+      if (r2 >= lo && r2 <= up)
+        open = exact_open(na, t.q[0], t.q[1], t.q[2], __int_as_float(nm.x & 0x7fffffff), th2d);
+      const int next = open ? (kSib ? nm.w : cur + 1) : nm.y;
+      go = --left > 0u && (unsigned)(next - root) < nn;
+      cur = go ? next : root;          // the last load is not used
+      const float mass = fabsf(na.w);  // cells carry their mass with the sign bit set
+      load_node(nodes, cur, na, nm);
+      const float rinv = rsqrt_normal(fmaxf(r2, 1e-30f));
+      float contrib = -mass * rinv;
+      if (r2 < h2f) contrib = softened_fp32(mass, r2, rinv, hf, hinvf);
+      contrib = open ? 0.f : contrib;
+      const float y = __fsub_rn(contrib, comp);
+      const float sum = __fadd_rn(hi, y);
+      comp = __fsub_rn(__fsub_rn(sum, hi), y);
+      hi = sum;
+      if (kGrad && !open) {
+        float w;  // gradient weight: grad phi -= m * w * dx
+        if (r2 >= h2f) {
+          w = rinv * rinv * rinv;
+        } else {
+          const float u = r2 * rinv * hinvf;
+          const float iu = hf * rinv;  // 1/u
+          const float dwp = u < 0.5f
+                                ? u * (10.666666666667f + u * u * (32.0f * u - 38.4f))
+                                : -0.066666666667f * iu * iu +
+                                      u * (21.333333333333f +
+                                           u * (-48.0f + u * (38.4f - 10.666666666667f * u)));
+          w = r2 > 0.f ? hinvf * hinvf * dwp * rinv : 0.f;
+        }
+        const float mw = mass * w;
+        kahan_add(ax, cx, mw * dx);
+        kahan_add(ay, cy, mw * dy);
+        kahan_add(az, cz, mw * dz);
       }
-      const float mw = mass * w;
-      kahan_add(ax, cx, mw * dx);
-      kahan_add(ay, cy, mw * dy);
-      kahan_add(az, cz, mw * dz);
-    }
-    iters++;
-    if (kSib) {
-      cur = open ? nm.w : nm.y;
-      if (iters >= steps || cur < t.nxt) break;  // malformed pointers: stop
-    } else {
-      cur = open ? cur + 1 : max(nm.y, cur + 1);
-    }
+    } while (go);
   }
   acc[0] = dsub((double)ax, (double)cx);
   acc[1] = dsub((double)ay, (double)cy);
