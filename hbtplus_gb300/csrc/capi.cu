@@ -431,6 +431,7 @@ void pass_tree_and_energies(Ctx &c, LoopHooks *hk)
 {
   const PassPlan pl = *c.plan_host;
   if (hk) hk->mark();
+  launch_list_order(c, pl);
   launch_tree_build(c, pl);
   if (hk) hk->mark();
   launch_walk(c, pl);

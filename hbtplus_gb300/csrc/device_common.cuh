@@ -245,18 +245,32 @@ void launch_bbox_cube(Ctx &c, int max_chunks);
 void launch_tree_build(Ctx &c, const PassPlan &pl);
 // launchers (walk.cu)
 void launch_walk(Ctx &c, const PassPlan &pl);
+// sorts the targets that come in list order, before the tree build
+void launch_list_order(Ctx &c, const PassPlan &pl);
 void launch_sibling_layout(Ctx &c, const PassPlan &pl);
+// Targets in list order are sorted along a space-filling curve (launch_list_order)
+// when a pass has at least kListMin of them: the sort's dozen launches take longer
+// than they save below (one subhalo of 7.2e4 particles, 1000 in the tree: the call
+// takes 1.20 ms without, 1.23 with; 2.4e5: 1.78 and 1.48), and when they are half of
+// the call's particles, all of which the sort moves.
+constexpr int kListMin = 1 << 17;
+inline bool list_order(const Ctx &c, const PassPlan &pl)
+{
+  return pl.nlist >= kListMin && pl.nlist >= c.N / 2;
+}
 // The FP32 lane walk of two neighbouring targets per lane (walk_pair): from
 // kPairMin targets on, 5 warps of pairs per scheduler.  Fewer lanes than that leave
 // the chip waiting on each walk's chain of loads (first pass of a subhalo of 1.1e5
 // particles: 937 us in pairs, 623 one by one; 1.6e5: 1014 and 967; 2.2e5: 1174 and
 // 1228; 3.4e5: 1607 and 2278; 1.1e6: 4.5 and 5.5 ms; 2.7e7: 122 and 160 ms).
-// Targets in list order are no neighbours: 780,000 of them took 810 us against 765.
+// Targets in list order are no neighbours: 780,000 of them took 810 us against 765,
+// sorted 607 against 637.
 // The gradient's walk stays with one target per lane.
 constexpr int kPairMin = 152 * 4 * 5 * 64;
 inline bool pair_walk(const Ctx &c, const PassPlan &pl)
 {
-  return c.P.precision != HBTU_PRECISION_FP64 && c.opt_schedule == 0 && pl.nlist == 0 &&
+  return c.P.precision != HBTU_PRECISION_FP64 && c.opt_schedule == 0 &&
+         (pl.nlist == 0 || list_order(c, pl)) &&
          pl.ntgt_total >= kPairMin && !(c.grad_pos || c.grad_vel || c.grad_mass);
 }
 // The FP32 lane walk over the sibling-block records (the tree build then makes

@@ -66,8 +66,8 @@ struct SegState {
   int t0, ntree, ntgt;
   float mfac;
   int nnodes;
-  int tgt_mode;         // 0 tree leaves (Morton), 1 last full pass's order, 2 list order
-  int coh_n;            // length of that Morton order
+  int tgt_mode;         // 0 tree leaves (Morton), 1 an earlier pass's order, 2 list order
+  int coh_n;            // length of that earlier order
   int ub_lo, ub_hi;     // list block removed by the last partition, to be sorted
   int refine;           // RefineBindingEnergyOrder pending (sampling, converged)
   int levels;
@@ -123,7 +123,8 @@ struct PassPlan {
   int nsort_total;  // elements of the unbound-part sort
   int nchunks_bound;
   int nrefine;
-  int norder, nlist;     // subhaloes whose targets follow an earlier pass's order, the list
+  int norder;            // subhaloes whose targets follow an earlier pass's order
+  int nlist;             // targets in list order
   int error;             // a sort's look-back wait ran out
   int max_nlast;         // longest energy list of an active subhalo
   long long inter_done;  // walk interactions summed so far, all subhaloes

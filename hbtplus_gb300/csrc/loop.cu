@@ -191,7 +191,7 @@ __device__ int get_pass(const Ctx &c, int s, int *v)
   const bool act = sg.status == SEG_ACTIVE;
   v[0] = act ? sg.ntree : 0;
   v[1] = act ? (sg.ntree + kChunk - 1) / kChunk : 0;
-  v[2] = act && sg.tgt_mode == 2;  // summed only
+  v[2] = act && sg.tgt_mode == 2 ? sg.ntgt : 0;  // summed only
   v[3] = sg.ub_hi - sg.ub_lo;
   return 0;
 }

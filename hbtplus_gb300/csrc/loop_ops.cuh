@@ -241,7 +241,7 @@ __device__ __forceinline__ void control_segment(const Ctx &c, SegState &sg, int 
     if (P.maxsample > 0 && nb > P.maxsample) {
       sg.ntree = (int)P.maxsample;
       sg.mfac = __fdiv_rn(__int2float_rn(nb), (float)P.maxsample);
-      sg.tgt_mode = 2;
+      sg.tgt_mode = sg.coh_n > 0 ? 1 : 2;
     } else {
       sg.ntree = nb;
       sg.mfac = 1.f;
