@@ -339,6 +339,11 @@ __device__ __forceinline__ Float2 f2_fma(Float2 a, Float2 b, Float2 c)
   return r;
 }
 
+struct PairSums {
+  Float2 hi, comp;  // Kahan sums
+  int ninter[2];
+};
+
 // FP32 walks of two neighbouring targets by one lane, over the union of the
 // nodes they visit (1.18 per node of one walk): each node is loaded once for
 // both.  A target that accepts a cell the other opens waits at the cell's skip
@@ -351,114 +356,97 @@ __device__ __forceinline__ Float2 f2_fma(Float2 a, Float2 b, Float2 c)
 // walk_lean's large launches wait for L1 (16.4 data wavefronts per load of 32
 // records, 84 to 90% of the cycles).  This loop takes 76 instructions per node of
 // the union against 2 x 49, 41% of the loads away, and issues on 72% of the cycles
-// at 67% of L1's wavefronts.  What made it pay: one 32-byte load per record, the
-// pairs of float operations in one instruction (distances and sums; the spline's
-// constants stay immediates, as pairs they cost 20 registers), the rare double
-// test and the near branch as loops, which the compiler does not predicate.
-// The next node's sibling-block record brought nothing here: a launch of 2.7e7
-// targets took 124 ms with them and 122 without, and their layout is not built.
+// at 67% of L1's wavefronts (79% of the sectors hit there); dropping a tenth of its
+// instructions did not change the time.  What made it pay: pairs of float operations
+// in one instruction (distances and sums; the spline's constants stay immediates, as
+// pairs they cost 20 registers), and the rare double test and the near branch as
+// loops, which the compiler does not predicate.  The sibling-block records brought
+// nothing here (2.7e7 targets: 124 ms with them, 122 without), and their layout is
+// not built.
 // With walk_grad's sums the same loop gained nothing (1e6 targets: 5.9 ms against
 // 5.7): 12 more registers and selects.
+//
+// The walks of those of t[0], t[1] with here[k], in the tree of nodes root .. end - 1.
 __device__ __forceinline__ void walk_pair(const WNode *nodes, const Target (&t)[2],
-                                          const DevParams &P, int (&ninter)[2], double (&pot)[2])
+                                          const bool (&here)[2], int root, int end,
+                                          const DevParams &P, PairSums &sums)
 {
-  const float zero[2] = {0.f, 0.f};
-  Float2 hi = f2_pack(zero), comp = hi;  // Kahan sums
-  bool todo[2] = {t[0].end > t[0].nxt, t[1].end > t[1].nxt};
-  ninter[0] = ninter[1] = 0;
-#pragma unroll 1
-  for (int first = 0; first < 2; first++) {  // targets of two subhaloes: one after the other
-    if (first == 0 ? !todo[0] : !todo[1]) continue;
-    const int root = first == 0 ? t[0].nxt : t[1].nxt;
-    const int end = first == 0 ? t[0].end : t[1].end;
-    int at[2];
+  int at[2] = {here[0] ? root : kDone, here[1] ? root : kDone};
+  Float2 hi = sums.hi, comp = sums.comp;
+  int cur = root;
+  float4 na;
+  int4 nm;
+  load_node(nodes, cur, na, nm);
+  bool go;
+  do {
+    bool open[2], vis[2];
+    float r2[2], neg[2], rinv[2], dx[2], dy[2], dz[2];
+    const int child = cur + 1, skip = max(nm.y, child);
+    const float lo = __int_as_float(nm.z), up = __int_as_float(nm.w);
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-      const bool here = todo[k] && t[k].nxt == root;
-      at[k] = here ? root : kDone;
-      todo[k] = todo[k] && !here;
+      dx[k] = na.x - t[k].q[0];
+      dy[k] = na.y - t[k].q[1];
+      dz[k] = na.z - t[k].q[2];
     }
-    int cur = root;
-    float4 na;
-    int4 nm;
-    load_node(nodes, cur, na, nm);
-    bool go;
-    do {
-      bool open[2], vis[2];
-      float r2[2], neg[2], rinv[2], dx[2], dy[2], dz[2];
-      const int child = cur + 1, skip = max(nm.y, child);
-      const float lo = __int_as_float(nm.z), up = __int_as_float(nm.w);
+    const Float2 x = f2_pack(dx), y = f2_pack(dy), z = f2_pack(dz);
+    f2_unpack(f2_fma(z, z, f2_fma(x, x, f2_mul(y, y))), r2);  // dist2
+#pragma unroll
+    for (int k = 0; k < 2; k++) open[k] = r2[k] < lo;
+    int band = (!open[0] && r2[0] <= up) || (!open[1] && r2[1] <= up);
+    while (__builtin_expect(band, 0)) {
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+        if (!open[k] && r2[k] <= up)
+          open[k] = opens_double(na, t[k].q[0], t[k].q[1], t[k].q[2],
+                                 __int_as_float(nm.x & 0x7fffffff), P.theta2d);
+      asm volatile("mov.u32 %0, 0;" : "=r"(band));
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      vis[k] = at[k] <= cur;
+      const bool take = vis[k] && !open[k];
+      neg[k] = take ? -fabsf(na.w) : 0.f;
+      if (take) {
+        sums.ninter[k]++;
+        at[k] = skip;
+      }
+    }
+    cur = (vis[0] && open[0]) || (vis[1] && open[1]) ? child : skip;
+    go = cur < end;
+    if (go) load_node(nodes, cur, na, nm);
+#pragma unroll
+    for (int k = 0; k < 2; k++) rinv[k] = rsqrt_normal(fmaxf(r2[k], 1e-30f));
+    Float2 contrib = f2_mul(f2_pack(neg), f2_pack(rinv));
+    int near = fminf(r2[0], r2[1]) < P.h2f;
+    while (near) {
+      float v[2];
+      f2_unpack(contrib, v);
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        dx[k] = na.x - t[k].q[0];
-        dy[k] = na.y - t[k].q[1];
-        dz[k] = na.z - t[k].q[2];
+        const float soft = softened_select(-neg[k], r2[k], rinv[k], P.hf, P.hinvf);
+        v[k] = r2[k] < P.h2f ? soft : v[k];
       }
-      const Float2 x = f2_pack(dx), y = f2_pack(dy), z = f2_pack(dz);
-      f2_unpack(f2_fma(z, z, f2_fma(x, x, f2_mul(y, y))), r2);  // dist2
+      contrib = f2_pack(v);
+      asm volatile("mov.u32 %0, 0;" : "=r"(near));
+    }
+    // an opened node adds zero, which can still settle the compensation
+    const Float2 add = f2_sub(contrib, comp), sum = f2_add(hi, add);
+    float h[2], c[2], s[2], e[2];
+    f2_unpack(hi, h);
+    f2_unpack(comp, c);
+    f2_unpack(sum, s);
+    f2_unpack(f2_sub(f2_sub(sum, hi), add), e);
 #pragma unroll
-      for (int k = 0; k < 2; k++) open[k] = r2[k] < lo;
-      int band = (!open[0] && r2[0] <= up) || (!open[1] && r2[1] <= up);
-      while (__builtin_expect(band, 0)) {
-#pragma unroll
-        for (int k = 0; k < 2; k++)
-          if (!open[k] && r2[k] <= up)
-            open[k] = opens_double(na, t[k].q[0], t[k].q[1], t[k].q[2],
-                                   __int_as_float(nm.x & 0x7fffffff), P.theta2d);
-        asm volatile("mov.u32 %0, 0;" : "=r"(band));
-      }
-#pragma unroll
-      for (int k = 0; k < 2; k++) {
-        vis[k] = at[k] <= cur;
-        const bool take = vis[k] && !open[k];
-        neg[k] = take ? -fabsf(na.w) : 0.f;
-        if (take) {
-          ninter[k]++;
-          at[k] = skip;
-        }
-      }
-      cur = (vis[0] && open[0]) || (vis[1] && open[1]) ? child : skip;
-      go = cur < end;
-      if (go) load_node(nodes, cur, na, nm);
-#pragma unroll
-      for (int k = 0; k < 2; k++) rinv[k] = rsqrt_normal(fmaxf(r2[k], 1e-30f));
-      Float2 contrib = f2_mul(f2_pack(neg), f2_pack(rinv));
-      int near = fminf(r2[0], r2[1]) < P.h2f;
-      while (near) {
-        float v[2];
-        f2_unpack(contrib, v);
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-          const float soft = softened_select(-neg[k], r2[k], rinv[k], P.hf, P.hinvf);
-          v[k] = r2[k] < P.h2f ? soft : v[k];
-        }
-        contrib = f2_pack(v);
-        asm volatile("mov.u32 %0, 0;" : "=r"(near));
-      }
-      // an opened node adds zero, which can still settle the compensation
-      const Float2 add = f2_sub(contrib, comp), sum = f2_add(hi, add);
-      float h[2], c[2], s[2], e[2];
-      f2_unpack(hi, h);
-      f2_unpack(comp, c);
-      f2_unpack(sum, s);
-      f2_unpack(f2_sub(f2_sub(sum, hi), add), e);
-#pragma unroll
-      for (int k = 0; k < 2; k++) {
-        h[k] = vis[k] ? s[k] : h[k];
-        c[k] = vis[k] ? e[k] : c[k];
-      }
-      hi = f2_pack(h);
-      comp = f2_pack(c);
-    } while (go);
-  }
-  float h[2], c[2];
-  f2_unpack(hi, h);
-  f2_unpack(comp, c);
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const double base = f2d(__fdiv_rn(t[k].mself, P.eps));  // cancels the self term
-    pot[k] = dadd(dadd(base, f2d(h[k])), -f2d(c[k]));
-  }
+    for (int k = 0; k < 2; k++) {
+      h[k] = vis[k] ? s[k] : h[k];
+      c[k] = vis[k] ? e[k] : c[k];
+    }
+    hi = f2_pack(h);
+    comp = f2_pack(c);
+  } while (go);
+  sums.hi = hi;
+  sums.comp = comp;
 }
 
 // The softened FP64 interaction with the reference's arithmetic, operation by operation
