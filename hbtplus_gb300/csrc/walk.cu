@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_count(Ctx c)
     if (lane == 31) c.pX[blockIdx.x] = x;
   }
   __syncthreads();
-  if (lane == 0) reinterpret_cast<uint2 *>(c.pcode)[p >> 5] = make_uint2(bits, wsum[w]);
+  if (lane == 0 && p < c.N)
+    reinterpret_cast<uint2 *>(c.pcode)[p >> 5] = make_uint2(bits, wsum[w]);
 }
 
 __global__ void __launch_bounds__(kWB) k_order_write(Ctx c)
