@@ -47,12 +47,13 @@ HBM_BYTES_PER_EVALUATION = 44  # read pos, vel, mass (28 B); write E and index (
 FP32_LANES_PER_SM = 128
 # DRAM bytes (read + write) of the first-pass walk launch, from one ncu capture of
 # the same workload (summaries in profiles/); None until captured for this kernel.
-WALK1_DRAM_BYTES = {"batch": 79971584}
-WALK1_PROFILE = {"batch": "walk_lean_pass1_batch2000.md"}
-# The same capture: the walk is limited by the L1 data path, not by DRAM or the FP32 pipe.
-WALK1_LIMITER = {"batch": "L1 data path: l1tex throughput 90% of peak at a 97% L1 hit rate, "
-                          "22 sectors per warp request (one 32-byte node record per lane per "
-                          "step; the lanes walk apart)"}
+WALK1_DRAM_BYTES = {"batch": 79253760}
+WALK1_PROFILE = {"batch": "walk_pair_pass1_batch2000.md"}
+# The same capture: not limited by DRAM or the FP32 pipe.
+WALK1_LIMITER = {"batch": "issue slots (71% of the cycles), the L1 data path (74% of its "
+                          "wavefronts) and the latency of L1 misses (21% of the sectors) "
+                          "together: the lanes walk apart"}
+PAIR_TARGETS = 194560  # launches of that many targets walk two per lane
 
 
 def parse():
@@ -697,11 +698,15 @@ def main():
     first_evals = ntot  # the first pass evaluates every particle once
     hbm_achieved = (first_evals * HBM_BYTES_PER_EVALUATION / (walk1_ms / 1e3) / 1e9
                     if walk1_ms else 0.0)
-    traffic = WALK1_DRAM_BYTES.get(args.workload) if args.precision == "fp32" else None
+    walk1_kernel = ("k_walk_fp64, one walk per lane" if args.precision == "fp64" else
+                    "k_walk_fp32" if args.walk_schedule == 1 else
+                    "k_walk_fp32_pair, two neighbouring walks per lane" if ntot >= PAIR_TARGETS
+                    else "k_walk_fp32_lean, one walk per lane")
+    captured = args.precision == "fp32" and args.walk_schedule != 1 and not args.max_sample
+    traffic = WALK1_DRAM_BYTES.get(args.workload) if captured else None
     roofline = {
-        "kernel": "k_walk_fp32_lean, first pass of the step (Barnes-Hut energy walk, one "
-                  "walk per lane, sibling-block node records)",
-        "limiter": WALK1_LIMITER.get(args.workload) if args.precision == "fp32" else None,
+        "kernel": walk1_kernel + ", first pass of the step (Barnes-Hut energy walk)",
+        "limiter": WALK1_LIMITER.get(args.workload) if captured else None,
         "bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
         "frac": achieved / fp32_peak if fp32_peak else None,
         "peak_source": f"{sm_count} SMs x {FP32_LANES_PER_SM} FP32 lanes x 2 flop at the "

@@ -355,8 +355,8 @@ struct PairSums {
 //
 // walk_lean's large launches wait for L1 (16.4 data wavefronts per load of 32
 // records, 84 to 90% of the cycles).  This loop takes 76 instructions per node of
-// the union against 2 x 49, 41% of the loads away, and issues on 72% of the cycles
-// at 67% of L1's wavefronts (79% of the sectors hit there); dropping a tenth of its
+// the union against 2 x 49, two fifths of the loads away, and issues on 71% of the
+// cycles at 74% of L1's wavefronts (79% of the sectors hit); dropping a tenth of its
 // instructions did not change the time.  What made it pay: pairs of float operations
 // in one instruction (distances and sums; the spline's constants stay immediates, as
 // pairs they cost 20 registers), and the rare double test and the near branch as
