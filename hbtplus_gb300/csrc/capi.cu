@@ -320,6 +320,10 @@ hbtu_status setup_call(hbtu_handle *h, const hbtu_particles *p, long long S, con
   c.opt_layout = (int)h->opt_layout;
   std::vector<int> order;
   order_by_size(offsets, S, nmax, order);
+  c.nlong = 0;
+  while (c.nlong < S && offsets[order[c.nlong] + 1] - offsets[order[c.nlong]] >
+                            (int64_t)(kLongSum - 1) * kChunk)
+    c.nlong++;
   // the per-subhalo loop takes over small subhaloes (small.cu); the walk of
   // its blocks is the default one-target-per-lane schedule
   c.small_cap = h->opt_schedule == 0 ? (int)std::min<int64_t>(h->opt_small, kSmallCap) : 0;

@@ -11,6 +11,9 @@
 namespace hbtu {
 
 constexpr int kChunk = 1024;  // elements per reduction chunk
+// Chunks from which on a subhalo's chunk sums are added by k_fold_chunks: with fewer,
+// the loop of sum_chunks (145 cycles a chunk) costs less than one more launch.
+constexpr int kLongSum = 64;
 constexpr int kDone = 0x7fffffff;
 
 // One tree node as the walks read it (32 bytes, one sector): p = {x, y, z,
@@ -238,6 +241,7 @@ struct Ctx {
   int *small_next;   // three work queues (large, medium, short lists): next jobs, counts, threads
   int *small_list;   // 3 S: their jobs, S each
   int small_cap;
+  int nlong;  // subhaloes whose chunk sums k_fold_chunks adds, the first of seg_order
 };
 
 // launchers (tree.cu)

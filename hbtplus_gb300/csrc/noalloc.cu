@@ -149,6 +149,7 @@ extern "C" hbtu_status hbtu_unbind_noalloc(const hbtu_params *params, const hbtu
     c.opt_schedule = 0;
     c.opt_layout = 0;
     c.small_cap = 0;  // every pass on the batch kernels
+    c.nlong = 0;      // at most 16 chunks
     SegState g;
     init_segment(g, 0, (int)n, *st, params->max_sample_size);
     const int segoff[2] = {0, (int)n};
