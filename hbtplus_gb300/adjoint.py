@@ -25,8 +25,9 @@ from . import _lib
 from .unbind import Unbinder, state_array
 
 
-def _states(ref_pos, ref_vel):
-    return state_array(ref_pos, ref_vel, ref_pos, ref_vel, np.full(len(ref_pos), -1, np.int64))
+def _states(nsub, ref_pos, ref_vel):
+    n = max(nsub, len(ref_pos))  # every row of ref_pos has its velocity
+    return state_array(n, ref_pos, ref_vel, ref_pos, ref_vel, np.full(n, -1, np.int64))
 
 
 def bound_subset(batch: dict, order, results) -> dict:
@@ -70,7 +71,7 @@ def energy_gradient(ub: Unbinder, pos: torch.Tensor, vel: torch.Tensor, mass: to
         gv = torch.empty((n, 3), dtype=torch.float32, device=dev)
         gm = torch.empty(n, dtype=torch.float32, device=dev)
         ptrs = [gp.data_ptr(), gv.data_ptr(), gm.data_ptr()]
-    sts = _states(np.asarray(ref_pos, np.float32), np.asarray(ref_vel, np.float32))
+    sts = _states(nsub, np.asarray(ref_pos, np.float32), np.asarray(ref_vel, np.float32))
     ub.set_stream(torch.cuda.current_stream(dev).cuda_stream)
     rc = ub.lib.hbtu_energy_gradient(ub.handle, C.byref(p), nsub, off.ctypes.data,
                                      C.addressof(sts), E.data_ptr(), *ptrs)

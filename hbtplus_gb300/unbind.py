@@ -186,17 +186,42 @@ def _host(values) -> np.ndarray:
     return values.detach().cpu().numpy() if hasattr(values, "detach") else np.asarray(values)
 
 
-def state_array(ref_pos, ref_vel, mostbound_pos, mostbound_vel, mostbound_id) -> C.Array:
-    """A ctypes array of hbtu_state, one per subhalo, from arrays of its fields."""
-    nsub = len(mostbound_id)
+def _field(values, nsub: int, width: int):
+    """The first nsub rows of one field of the states (width 0: one number a row, else
+    the first `width` of its columns), or None where values has another shape or
+    holds anything but ordinary numbers."""
+    try:
+        v = _host(values)
+    except (TypeError, ValueError):  # rows of unlike lengths or on a device, half types
+        return None
+    if v.dtype.kind not in ("iuf" if width else "iu") or v.dtype.itemsize > 8 or len(v.shape) != (
+            2 if width else 1) or len(v) < nsub or (width and v.shape[1] < width):
+        return None
+    # a coordinate becomes a double before a float, as float() makes it
+    return v[:nsub, :width].astype(np.float64) if width else v[:nsub]
+
+
+def state_array(nsub: int, ref_pos, ref_vel, mostbound_pos, mostbound_vel, mostbound_id) -> C.Array:
+    """A ctypes array of nsub hbtu_state from the fields' rows 0 .. nsub - 1: at once
+    where every field is a table of numbers with at least that many rows, otherwise
+    row by row, which takes whatever indexing and float() take and raises where a row
+    or a coordinate is missing."""
     sts = (_lib.hbtu_state * max(nsub, 1))()
+    if nsub <= 0:
+        return sts
+    fields = dict(ref_pos=_field(ref_pos, nsub, 3), ref_vel=_field(ref_vel, nsub, 3),
+                  mostbound_pos=_field(mostbound_pos, nsub, 3),
+                  mostbound_vel=_field(mostbound_vel, nsub, 3),
+                  mostbound_id=_field(mostbound_id, nsub, 0))
+    if any(v is None for v in fields.values()):
+        for s in range(nsub):
+            sts[s] = _state(ref_pos[s], ref_vel[s], mostbound_pos[s], mostbound_vel[s],
+                            mostbound_id[s])
+        return sts
     rec = np.frombuffer(sts, dtype=np.dtype(_lib.hbtu_state), count=nsub)
-    for name, values in (("ref_pos", ref_pos), ("ref_vel", ref_vel),
-                         ("mostbound_pos", mostbound_pos), ("mostbound_vel", mostbound_vel),
-                         ("mostbound_id", mostbound_id)):
-        if nsub:
-            v = _host(values)
-            rec[name] = v[:nsub, :3] if v.ndim > 1 else v[:nsub]
+    with np.errstate(over="ignore"):  # beyond the floats: infinite
+        for name, v in fields.items():
+            rec[name] = v
     return sts
 
 
@@ -437,13 +462,13 @@ class Unbinder:
         off = np.asarray(_host(batch["offsets"]), np.int64)
         nsub = len(off) - 1
         if "mostbound_id" in batch:
-            mb_id = _host(batch["mostbound_id"])[:nsub]
+            mb_id = batch["mostbound_id"]
         else:  # each list's first particle
             ids = _host(batch["id"])
-            mb_id = np.full(nsub, -1, np.int64)
+            mb_id = np.full(max(nsub, 0), -1, np.int64)
             some = off[1:] > off[:-1]
             mb_id[some] = ids[off[:-1][some]]
-        return state_array(batch["ref_pos"], batch["ref_vel"], batch["mostbound_pos"],
+        return state_array(nsub, batch["ref_pos"], batch["ref_vel"], batch["mostbound_pos"],
                            batch["mostbound_vel"], mb_id)
 
 
