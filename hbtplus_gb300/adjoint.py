@@ -26,6 +26,8 @@ from .unbind import Unbinder, state_array
 
 
 def _states(nsub, ref_pos, ref_vel):
+    if nsub == 1:  # one subhalo's frame may come as a bare triple
+        ref_pos, ref_vel = (v[None] if v.ndim == 1 else v for v in (ref_pos, ref_vel))
     n = max(nsub, len(ref_pos))  # every row of ref_pos has its velocity
     return state_array(n, ref_pos, ref_vel, ref_pos, ref_vel, np.full(n, -1, np.int64))
 

@@ -60,6 +60,14 @@ def test_gradient_frames_are_refused(shape):
     assert len(adjoint._states(4, whole, whole)) >= 4
 
 
+def test_gradient_of_one_subhalo_takes_a_triple():
+    x, v = np.arange(3, dtype=np.float32), np.arange(3, 6, dtype=np.float32)
+    assert bytes(adjoint._states(1, x, v)) == bytes(adjoint._states(1, x[None], v[None]))
+    for a, b in ((x[:2], v), (x, v[:1])):
+        with pytest.raises((IndexError, TypeError)):
+            adjoint._states(1, a, b)
+
+
 FORMS = {
     "float64": lambda v: v.astype(np.float64) * (1 + 1e-9),
     "integers": lambda v: (v * 1e16).astype(np.int64),
