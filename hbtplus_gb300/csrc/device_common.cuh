@@ -40,6 +40,12 @@ __device__ __forceinline__ void load_node(const WNode *nd, int i, float4 &p, int
   m = make_int2(q.x, q.y);
 }
 
+// First octant slot of the cell of element e (Ctx::cslot) and first coordinate of particle
+// i in an array of triples: a call holds up to 2^30 of them, and an int's product
+// overflows from 2^28 and 2^31 / 3 on.
+__host__ __device__ inline size_t first_slot(int e) { return 8 * (size_t)e; }
+__host__ __device__ inline size_t first_coord(int i) { return 3 * (size_t)i; }
+
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }

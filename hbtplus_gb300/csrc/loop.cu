@@ -170,8 +170,9 @@ __global__ void k_init(Ctx c, const float *pos, const float *vel, const float *m
   if (i >= c.N) return;
   const int s = upper_bound_i(c.seg_off, c.S + 1, i) - 1;
   c.pseg[i] = s;
-  c.pm[i] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], mass[i]);
-  c.vel[i] = make_float4(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2], 0.f);
+  const float *x = pos + first_coord(i), *v = vel + first_coord(i);
+  c.pm[i] = make_float4(x[0], x[1], x[2], mass[i]);
+  c.vel[i] = make_float4(v[0], v[1], v[2], 0.f);
   c.epid[i] = i;
   c.eE[i] = 0.f;
   c.epos_of_pid[i] = i;

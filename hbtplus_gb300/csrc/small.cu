@@ -269,7 +269,7 @@ __device__ __forceinline__ ull *tree_keys(const Group &g, const Ctx &c, int P0)
     const int e = P0 + i;
     c.mask[e] = 0ull;
     c.pending[e] = 0;
-    int4 *slot = reinterpret_cast<int4 *>(c.cslot + 8 * (size_t)e);
+    int4 *slot = reinterpret_cast<int4 *>(c.cslot + first_slot(e));
     slot[0] = make_int4(-1, -1, -1, -1);
     slot[1] = make_int4(-1, -1, -1, -1);
   }

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kTB) k_keys(Ctx c, int ntotal)
   c.mask[e] = 0ull;
   c.pending[e] = 0;
   c.pending0[e] = 0;
-  int4 *slot = reinterpret_cast<int4 *>(c.cslot + 8 * (size_t)e);
+  int4 *slot = reinterpret_cast<int4 *>(c.cslot + first_slot(e));
   slot[0] = make_int4(-1, -1, -1, -1);
   slot[1] = make_int4(-1, -1, -1, -1);
   const int s = upper_bound_i(c.tree_base, c.S + 1, e) - 1;
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_moments_chunks(Ctx c)
         const int d = c.cdepth[e];
         if (d >= 0) {
           const int r = min(max(d - d0, 0), kDepthBins - 1);
-          const int4 *slot = reinterpret_cast<const int4 *>(c.cslot + 8 * e);
+          const int4 *slot = reinterpret_cast<const int4 *>(c.cslot + first_slot(e));
           const int4 a = slot[0], b = slot[1];
           const int kids = (a.x >= 0) + (a.y >= 0) + (a.z >= 0) + (a.w >= 0) + (b.x >= 0) +
                            (b.y >= 0) + (b.z >= 0) + (b.w >= 0);
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kChunkThreads) k_moments_chunks(Ctx c)
       q.end = c.cskip[e];
       q.bucket = c.cdepth[e] >= sg.levels;
       q.mark = c.pending[e] == 0;
-      const int4 *slot = reinterpret_cast<const int4 *>(c.cslot + 8 * e);
+      const int4 *slot = reinterpret_cast<const int4 *>(c.cslot + first_slot(e));
       q.s0 = slot[0];
       q.s1 = slot[1];
       q.fc[0] = sg.fc[0];
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(kTB) k_sib_count(Ctx c, int ntotal)
   int k = 0;
   if (c.cdepth[e] < c.seg[s].levels) {
     for (int j = 0; j < 8; j++) {
-      const int sl = c.cslot[8 * e + j];
+      const int sl = c.cslot[first_slot(e) + j];
       k += (sl > idx && sl < end);
     }
   } else {  // a bucket: its particles follow it, one after another
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(kTB) k_sib_assign(Ctx c, int ntotal)
   int k = 0;
   if (c.cdepth[e] < c.seg[s].levels) {
     for (int j = 0; j < 8; j++) {
-      const int sl = c.cslot[8 * e + j];
+      const int sl = c.cslot[first_slot(e) + j];
       if (sl > idx && sl < end) c.newidx[sl] = base + k++;
     }
   } else {

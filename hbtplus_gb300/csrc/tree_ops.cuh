@@ -336,7 +336,7 @@ __device__ __forceinline__ void leaves_elem(const Ctx &c, SegState &sg, int base
   for (int guard = 0; p >= 0 && !c.iscell[p] && guard < 256; guard++) p = c.parentI[p];
   if (p >= 0 && c.iscell[p]) {
     const int odp = oct_depth(c.dnode[p], sg.levels);
-    if (odp < sg.levels) c.cslot[8 * p + octant_at(key, odp + 1)] = nb + idx;
+    if (odp < sg.levels) c.cslot[first_slot(p) + octant_at(key, odp + 1)] = nb + idx;
   }
 }
 
@@ -368,7 +368,7 @@ __device__ __forceinline__ void cellnodes_elem(const Ctx &c, const SegState &sg,
   if (p >= 0) {
     atomicAdd(&c.pending[p], 1);
     const int odp = oct_depth(c.dnode[p], sg.levels);
-    c.cslot[8 * p + octant_at(keys[lo], odp + 1)] = nb + idx;
+    c.cslot[first_slot(p) + octant_at(keys[lo], odp + 1)] = nb + idx;
   }
 }
 
@@ -494,7 +494,7 @@ __device__ __forceinline__ float4 cell_moment_of(const Ctx &c, const SegState &s
   int4 s0 = make_int4(-1, -1, -1, -1), s1 = s0;
   const bool bucket = depth >= sg.levels;
   if (!bucket) {
-    const int4 *slot = reinterpret_cast<const int4 *>(c.cslot + 8 * e);
+    const int4 *slot = reinterpret_cast<const int4 *>(c.cslot + first_slot(e));
     s0 = kCG ? __ldcg(slot) : slot[0];
     s1 = kCG ? __ldcg(slot + 1) : slot[1];
   }

@@ -489,9 +489,10 @@ __device__ __forceinline__ void finish_grad(const Ctx &c, const Target &t, doubl
   const int i = t.pid;  // no list permutation in this call: input position
   if (kGrad) {
     if (c.grad_pos)
-      for (int j = 0; j < 3; j++) c.grad_pos[3 * i + j] = (float)(m * (ha * dv[j] - ga * acc[j]));
+      for (int j = 0; j < 3; j++)
+        c.grad_pos[first_coord(i) + j] = (float)(m * (ha * dv[j] - ga * acc[j]));
     if (c.grad_vel)
-      for (int j = 0; j < 3; j++) c.grad_vel[3 * i + j] = (float)(m * dv[j]);
+      for (int j = 0; j < 3; j++) c.grad_vel[first_coord(i) + j] = (float)(m * dv[j]);
     if (c.grad_mass) c.grad_mass[i] = (float)(0.5 * k2 + pot);
   }
   c.e_part[i] = 0.5 * m * k2 + 0.5 * m * pot;
