@@ -472,6 +472,18 @@ static __device__ __noinline__ double fp64_contrib_any(double r2, double mass, d
   return fp64_softened(r, mass, h_inv);
 }
 
+// Whether a correction x / y, taken with a reciprocal of y good to a few units in the last
+// place, may have rounded the corrected value the wrong way: only where x / y is within
+// 2^-46 of half a unit of that value, a power of two, so where the mantissas of x and y
+// agree to 64 units.  (The bits of x = 0 count as mantissa zero: then exact, and
+// perhaps reported.)
+__device__ __forceinline__ bool near_half(double x, double y)
+{
+  const unsigned long long d =
+      (unsigned long long)__double_as_longlong(x) - (unsigned long long)__double_as_longlong(y);
+  return ((d + 64ull) & 0xfffffffffffffull) <= 128ull;
+}
+
 // The interaction at squared distance r2: -mass / r outside the softening length, r
 // the rounded root, both operations correctly rounded as the reference's are.
 // Root and reciprocal together, from one float approximation of 1/sqrt(r2): the
@@ -479,8 +491,12 @@ static __device__ __noinline__ double fp64_contrib_any(double r2, double mass, d
 // corrected by its exact remainder, and the quotient from 2k corrected twice by
 // its own (Markstein 1990; Cornea, Harrison & Tang 2002): 14 double operations, where
 // the two library operations took about 20 of the FP64 pipe, which is what
-// bounds this walk.  Outside the range where no step can leave the normal
-// doubles or floats, the library operations.
+// bounds this walk.  The corrections are taken with k, not with a correctly rounded
+// reciprocal, so a root or quotient within 2^-50 of a unit of the midpoint of two
+// doubles could fall on its other side (58 of 1622 quotients built to lie that close
+// did); where the last remainder says that it may be (near_half: integer code),
+// and outside the range where no step can leave the normal doubles or floats,
+// the library operations.
 __device__ __forceinline__ double fp64_contrib(double r2, float mass, const DevParams &P)
 {
   const unsigned ex = (unsigned)((unsigned long long)__double_as_longlong(r2) >> 52);
@@ -495,14 +511,18 @@ __device__ __forceinline__ double fp64_contrib(double r2, float mass, const DevP
   e = __fma_rn(-g, k, 0.5);
   g = __fma_rn(g, e, g);
   k = __fma_rn(k, e, k);
-  const double r = __fma_rn(__fma_rn(-g, g, r2), k, g);
+  const double rem = __fma_rn(-g, g, r2);  // r = g + rem / 2g
+  const double r = __fma_rn(rem, k, g);
   const double m = f2d(mass);
   // positive doubles compare as their bits do
-  if (__double_as_longlong(r) < __double_as_longlong(P.h)) return fp64_softened(r, m, P.h_inv);
+  if (__double_as_longlong(r) < __double_as_longlong(P.h) && !near_half(rem, g))
+    return fp64_softened(r, m, P.h_inv);
   const double inv = __longlong_as_double(__double_as_longlong(k) + (1ll << 52));
   double q = dmul(m, inv);
   q = __fma_rn(__fma_rn(-q, r, m), inv, q);
-  return -__fma_rn(__fma_rn(-q, r, m), inv, q);
+  const double qrem = __fma_rn(-q, r, m);
+  if (near_half(rem, g) || near_half(qrem, r)) return fp64_contrib_any(r2, m, P.h, P.h_inv);
+  return -__fma_rn(qrem, inv, q);
 }
 
 // r^2 of a collected node (walk_fp64).
