@@ -57,10 +57,11 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 // Exact float -> double and round-to-nearest-even double -> float, built
 // from the IEEE-754 fields with integer operations: the conversion
 // instructions run on the FP64 unit, at 1/64 of the FP32 rate on this GPU.
-// The special cases are integer code too.  A double instruction behind a
-// condition is no way out: the compiler predicates short branches, and a
-// predicated-off double instruction holds the FP64 unit as long as an executed
-// one (measured: 20 of them per step in a walk took it from 1.5 to 25 ms).
+// The special cases are integer code too; the results are the instructions', bit for
+// bit (f2d leaves it to the next operation to quiet a signalling NaN).  A double
+// instruction behind a condition is no way out: the compiler predicates short
+// branches, and a predicated-off double instruction holds the FP64 unit as long as
+// an executed one (measured: 20 of them per step in a walk took it from 1.5 to 25 ms).
 // Rare double paths in this library are calls for the same reason.
 __device__ __forceinline__ double f2d(float x)
 {
@@ -90,8 +91,8 @@ __device__ __forceinline__ float d2f(double x)
     const unsigned long long m = mant | (1ull << 52);
     const unsigned long long q = m >> s, rem = m & ((1ull << s) - 1ull), half = 1ull << (s - 1);
     bits = s > 53 ? 0u : (unsigned)q + (rem + (q & 1ull) > half ? 1u : 0u);
-  } else if (e >= 255 || bits >= 0x7f800000u) {  // overflow, infinity or NaN
-    bits = e == 0x7ff - 1023 + 127 && mant ? 0x7fc00000u : 0x7f800000u;
+  } else if (e >= 255 || bits >= 0x7f800000u) {  // overflow, infinity or NaN (quiet, payload kept)
+    bits = e == 0x7ff - 1023 + 127 && mant ? 0x7fc00000u | (unsigned)(mant >> 29) : 0x7f800000u;
   }
   return __uint_as_float(bits | ((unsigned)(b >> 63) << 31));
 }

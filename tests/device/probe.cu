@@ -7,6 +7,22 @@ using namespace hbtu;
 
 namespace {
 
+__global__ void k_f2d(const float *x, int n, double *got, double *want)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  got[i] = f2d(x[i]);
+  want[i] = (double)x[i];
+}
+
+__global__ void k_d2f(const double *x, int n, float *got, float *want)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  got[i] = d2f(x[i]);
+  want[i] = __double2float_rn(x[i]);
+}
+
 __global__ void k_fp64_contrib(const double *r2, const float *m, int n, DevParams P, double *got,
                                double *want)
 {
@@ -54,6 +70,22 @@ DevParams softening_params(double h)
 }  // namespace
 
 extern "C" {
+
+int probe_f2d(const float *x, int n, double *got, double *want)
+{
+  return run(x, (const float *)nullptr, n, got, want,
+             [&](int nb, float *dx, float *, double *g, double *w) {
+               k_f2d<<<nb, 128>>>(dx, n, g, w);
+             });
+}
+
+int probe_d2f(const double *x, int n, float *got, float *want)
+{
+  return run(x, (const float *)nullptr, n, got, want,
+             [&](int nb, double *dx, float *, float *g, float *w) {
+               k_d2f<<<nb, 128>>>(dx, n, g, w);
+             });
+}
 
 int probe_fp64_contrib(const double *r2, const float *m, int n, double h, double *got, double *want)
 {
