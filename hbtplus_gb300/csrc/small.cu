@@ -856,15 +856,25 @@ int resident_blocks()
   return 2 * sms;
 }
 
+// Shared memory of a block, for lists of up to `cap`, with or without large ones.
+size_t block_bytes(int cap, bool large)
+{
+  const size_t quads = (kSB / kMT) * quad_bytes(cap);
+  return large ? std::max(quads, SmallLayout(cap).bytes) : quads;
+}
+
 // n[k]: upper bounds of the jobs of each class.
 void launch(Ctx &c, const SmallCall &io, int whole, const SmallJobs &jobs, int cap,
             const int (&n)[3], int max_passes)
 {
-  size_t smem = (kSB / kMT) * quad_bytes(cap);
-  if (n[0] > 0) smem = std::max(smem, SmallLayout(cap).bytes);
+  const size_t smem = block_bytes(cap, n[0] > 0);
   void (*kernel)(Ctx, SmallCall, SmallJobs, int, int, int) =
       c.P.precision == HBTU_PRECISION_FP64 ? k_unbind_small<true> : k_unbind_small<false>;
-  HBTU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // The attribute is the kernel's, not the launch's: set to what a call's own lists need, it
+  // could fall below another thread's need between that thread's setting and
+  // its launch.  Every call sets the largest.
+  HBTU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)block_bytes(kSmallCap, true)));
   const int resident = resident_blocks();
   // few large lists: a cluster of blocks each, while half the chip holds them and
   // each block has a warp per scheduler
