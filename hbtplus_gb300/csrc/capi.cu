@@ -224,29 +224,19 @@ void order_by_size(const int64_t *offsets, long long S, long long nmax, std::vec
 }
 
 // A call whose subhaloes are all small enough (small.cu): its input besides the
-// particles goes to the device in one copy from a pinned buffer.
+// particles goes to the device in one copy.
 hbtu_status stage_small_call(hbtu_handle *h, long long S, const int64_t *offsets,
                              const hbtu_state *st, const std::vector<int> &order, Ctx &c,
                              Staging &sg, SmallCall &io)
 {
   const size_t bytes = call_bytes(S);
-  if (bytes > h->pin_bytes) {
-    if (h->pin) cudaFreeHost(h->pin);
-    h->pin = nullptr;
-    h->pin_bytes = 0;
-    if (cudaMallocHost(&h->pin, bytes + bytes / 4) != cudaSuccess) {
-      cudaGetLastError();
-      h->pin = nullptr;
-      return fail(h, HBTU_ERR_OUT_OF_MEMORY, "pinned staging buffer");
-    }
-    h->pin_bytes = bytes + bytes / 4;
-  }
+  char *buf = h->call_input.reserve(bytes);
   int T[3];
   small_classes(offsets, order.data(), (int)S, io.jobs, T);
   const int queue[10] = {0, 0, 0, io.jobs[0], io.jobs[1], io.jobs[2], T[0], T[1], T[2], 0};
   size_t o = 0;
   auto put = [&](const void *src, size_t n) {
-    memcpy(h->pin + o, src, n);
+    memcpy(buf + o, src, n);
     char *dev = sg.call + o;
     o += n;
     return dev;
@@ -255,7 +245,7 @@ hbtu_status stage_small_call(hbtu_handle *h, long long S, const int64_t *offsets
   io.off = (const long long *)put(offsets, sizeof(long long) * (S + 1));
   io.st = (const hbtu_state *)put(st, sizeof(hbtu_state) * S);
   io.order = (const int *)put(order.data(), sizeof(int) * S);
-  HBTU_CUDA(cudaMemcpyAsync(sg.call, h->pin, bytes, cudaMemcpyHostToDevice, c.st));
+  HBTU_CUDA(cudaMemcpyAsync(sg.call, buf, bytes, cudaMemcpyHostToDevice, c.st));
   return HBTU_OK;
 }
 
@@ -599,7 +589,7 @@ hbtu_status hbtu_destroy(hbtu_handle *h)
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->ws) cudaFree(h->ws);
   if (h->plan_host) cudaFreeHost(h->plan_host);
-  if (h->pin) cudaFreeHost(h->pin);
+  h->call_input.release();
   for (cudaEvent_t e : h->events) cudaEventDestroy(e);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   delete h;

@@ -7,6 +7,36 @@
 
 #include "device_common.cuh"
 
+namespace hbtu {
+// Host memory that a call's input is gathered in before its copy: pinned, or ordinary
+// memory where no pinned memory can be had (the copy is then staged by the driver).
+struct HostStaging {
+  char *reserve(size_t bytes)
+  {
+    if (bytes <= size) return pinned;
+    release();
+    const size_t want = bytes + bytes / 4;
+    if (cudaMallocHost(&pinned, want) == cudaSuccess) {
+      size = want;
+      return pinned;
+    }
+    cudaGetLastError();
+    pinned = nullptr;
+    plain.resize(bytes);
+    return plain.data();
+  }
+  void release()
+  {
+    if (pinned) cudaFreeHost(pinned);
+    pinned = nullptr;
+    size = 0;
+  }
+  char *pinned = nullptr;
+  size_t size = 0;
+  std::vector<char> plain;
+};
+}  // namespace hbtu
+
 struct hbtu_handle {
   hbtu_params params;
   hbtu::DevParams dp;
@@ -16,8 +46,7 @@ struct hbtu_handle {
   char *ws = nullptr;
   size_t ws_bytes = 0;
   hbtu::PassPlan *plan_host = nullptr;
-  char *pin = nullptr;  // pinned staging of a call's offsets, states and order
-  size_t pin_bytes = 0;
+  hbtu::HostStaging call_input;  // a call's offsets, states and order
   // tracing
   hbtu_stats stats{};
   bool timing = false;
