@@ -186,6 +186,17 @@ def _host(values) -> np.ndarray:
     return values.detach().cpu().numpy() if hasattr(values, "detach") else np.asarray(values)
 
 
+def _rows(values, rows) -> np.ndarray:
+    """Those rows of values (as for _host) as a numpy array; of a tensor only they leave its
+    device."""
+    if not hasattr(values, "detach"):
+        return np.asarray(values)[rows]
+    if len(rows) and (rows.max() >= len(values) or rows.min() < -len(values)):
+        raise IndexError("row out of range")  # on the host: a device would fault
+    import torch
+    return _host(values[torch.as_tensor(rows, device=values.device)])
+
+
 def _field(values, nsub: int, width: int):
     """The first nsub rows of one field of the states (width 0: one number a row, else
     the first `width` of its columns), or None where values has another shape or
@@ -464,10 +475,9 @@ class Unbinder:
         if "mostbound_id" in batch:
             mb_id = batch["mostbound_id"]
         else:  # each list's first particle
-            ids = _host(batch["id"])
             mb_id = np.full(max(nsub, 0), -1, np.int64)
             some = off[1:] > off[:-1]
-            mb_id[some] = ids[off[:-1][some]]
+            mb_id[some] = _rows(batch["id"], off[:-1][some])
         return state_array(nsub, batch["ref_pos"], batch["ref_vel"], batch["mostbound_pos"],
                            batch["mostbound_vel"], mb_id)
 

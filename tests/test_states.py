@@ -106,3 +106,19 @@ def test_ids_default_to_each_lists_first(nsub):
     del b["mostbound_id"]
     got = Unbinder.make_states(b)
     assert bytes(got)[:C.sizeof(_lib.hbtu_state) * nsub] == want
+
+
+def test_only_the_lists_first_ids_are_copied(monkeypatch):
+    from hbtplus_gb300 import unbind
+    b = _batch(seed=4)
+    del b["mostbound_id"]
+    want = bytes(Unbinder.make_states(b))
+    copied = []
+    host = unbind._host
+    monkeypatch.setattr(unbind, "_host", lambda v: copied.append(len(v)) or host(v))
+    b["id"] = torch.from_numpy(b["id"].copy())
+    assert bytes(Unbinder.make_states(b)) == want
+    assert len(b["id"]) > 6 and max(copied) <= 6
+    b["offsets"] = b["offsets"] + len(b["id"])
+    with pytest.raises(IndexError):
+        Unbinder.make_states(b)
