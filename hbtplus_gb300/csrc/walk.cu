@@ -188,6 +188,14 @@ __global__ void __launch_bounds__(kWB) k_list_write(Ctx c)
   c.epid2[p] = c.epid[c.sb.val_a[p]];
 }
 
+// The warp schedule's squared distance: with the compiler's own choice of fused
+// multiply-adds, which is not dist2's (the lane schedule's) everywhere.
+__device__ __forceinline__ float dist2_warp(float4 na, const float q[3])
+{
+  const float dx = na.x - q[0], dy = na.y - q[1], dz = na.z - q[2];
+  return dx * dx + dy * dy + dz * dz;
+}
+
 // FP32 walk, warp schedule.  Leaf runs: when targets open a cell
 // whose children are all particles, each of those targets takes every child
 // in order (particles are never opened) -- the warp streams the children
@@ -222,7 +230,7 @@ __global__ void __launch_bounds__(kWB) k_walk_fp32(Ctx c, int total)
     const int sk = nm.y;
     bool run = false;
     if (t.nxt == cur) {
-      const float r2 = dist2(na, t.q);
+      const float r2 = dist2_warp(na, t.q);
       if (opens(na, t.q, l2, r2, theta2, th2d)) {
         if (bottom)
           run = true;
@@ -243,13 +251,13 @@ __global__ void __launch_bounds__(kWB) k_walk_fp32(Ctx c, int total)
       for (; j + 1 < last; j += 2) {
         const float4 a0 = c.nd[j].p, a1 = c.nd[j + 1].p;
         if (run) {
-          interact(a0, dist2(a0, t.q), acc.f, hf, h2f, hinvf);
-          interact(a1, dist2(a1, t.q), acc.f, hf, h2f, hinvf);
+          interact(a0, dist2_warp(a0, t.q), acc.f, hf, h2f, hinvf);
+          interact(a1, dist2_warp(a1, t.q), acc.f, hf, h2f, hinvf);
         }
       }
       if (j < last) {
         const float4 a0 = c.nd[j].p;
-        if (run) interact(a0, dist2(a0, t.q), acc.f, hf, h2f, hinvf);
+        if (run) interact(a0, dist2_warp(a0, t.q), acc.f, hf, h2f, hinvf);
       }
       if (run) {
         ninter += last - cur - 1;
