@@ -212,6 +212,11 @@ def _field(values, nsub: int, width: int):
     return v[:nsub, :width].astype(np.float64) if width else v[:nsub]
 
 
+# Up to this many subhaloes the rows are taken one by one: 3 to 7 us each, where the tables take
+# 20 to 30 us together.  (Not of tensors: each number of a device tensor is a copy of its own.)
+_FEW_STATES = 4
+
+
 def state_array(nsub: int, ref_pos, ref_vel, mostbound_pos, mostbound_vel, mostbound_id) -> C.Array:
     """A ctypes array of nsub hbtu_state from the fields' rows 0 .. nsub - 1: at once
     where every field is a table of numbers with at least that many rows, otherwise
@@ -220,11 +225,13 @@ def state_array(nsub: int, ref_pos, ref_vel, mostbound_pos, mostbound_vel, mostb
     sts = (_lib.hbtu_state * max(nsub, 1))()
     if nsub <= 0:
         return sts
-    fields = dict(ref_pos=_field(ref_pos, nsub, 3), ref_vel=_field(ref_vel, nsub, 3),
-                  mostbound_pos=_field(mostbound_pos, nsub, 3),
-                  mostbound_vel=_field(mostbound_vel, nsub, 3),
-                  mostbound_id=_field(mostbound_id, nsub, 0))
-    if any(v is None for v in fields.values()):
+    given = dict(ref_pos=ref_pos, ref_vel=ref_vel, mostbound_pos=mostbound_pos,
+                 mostbound_vel=mostbound_vel, mostbound_id=mostbound_id)
+    if nsub <= _FEW_STATES and not any(hasattr(v, "detach") for v in given.values()):
+        fields = {}
+    else:
+        fields = {k: _field(v, nsub, 0 if k == "mostbound_id" else 3) for k, v in given.items()}
+    if not fields or any(v is None for v in fields.values()):
         for s in range(nsub):
             sts[s] = _state(ref_pos[s], ref_vel[s], mostbound_pos[s], mostbound_vel[s],
                             mostbound_id[s])

@@ -122,3 +122,11 @@ def test_only_the_lists_first_ids_are_copied(monkeypatch):
     b["offsets"] = b["offsets"] + len(b["id"])
     with pytest.raises(IndexError):
         Unbinder.make_states(b)
+
+
+@pytest.mark.parametrize("nsub", [1, 4, 5])
+def test_few_and_many_states_are_the_same(nsub):
+    b = _batch(nsub, seed=6)
+    assert bytes(Unbinder.make_states(b)) == _by_row(b)
+    tensors = {k: torch.from_numpy(v.copy()) if k in FRAMES else v for k, v in b.items()}
+    assert bytes(Unbinder.make_states(tensors)) == _by_row(b)
