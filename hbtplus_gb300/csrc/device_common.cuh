@@ -259,6 +259,12 @@ void launch_walk(Ctx &c, const PassPlan &pl);
 // sorts the targets that come in list order, before the tree build
 void launch_list_order(Ctx &c, const PassPlan &pl);
 void launch_sibling_layout(Ctx &c, const PassPlan &pl);
+// The FP32 walk's warp schedule sums a target's terms in parts that depend on the warp's other
+// targets: its passes take them as they come, without the orders below.
+__host__ __device__ inline bool warp_schedule(const Ctx &c)
+{
+  return c.opt_schedule == 1 && c.P.precision != HBTU_PRECISION_FP64;
+}
 // Targets in list order are sorted along a space-filling curve (launch_list_order)
 // when a pass has at least kListMin of them: the sort's dozen launches take longer
 // than they save below (one subhalo of 7.2e4 particles, 1000 in the tree: the call
@@ -267,7 +273,7 @@ void launch_sibling_layout(Ctx &c, const PassPlan &pl);
 constexpr int kListMin = 1 << 17;
 inline bool list_order(const Ctx &c, const PassPlan &pl)
 {
-  return pl.nlist >= kListMin && pl.nlist >= c.N / 2;
+  return pl.nlist >= kListMin && pl.nlist >= c.N / 2 && !warp_schedule(c);
 }
 // The FP32 lane walk of two neighbouring targets per lane (walk_pair): from
 // kPairMin targets on, 5 warps of pairs per scheduler.  Fewer lanes than that leave

@@ -196,14 +196,16 @@ __device__ int get_pass(const Ctx &c, int s, int *v)
   v[3] = sg.ub_hi - sg.ub_lo;
   return 0;
 }
-// targets of the pass, subhaloes in size order (largest first)
+// targets of the pass, subhaloes in size order (largest first); the warp schedule's correction
+// passes keep the places of the particles removed since the last full pass
 __device__ int get_targets_sorted(const Ctx &c, int k, int *v)
 {
   const SegState &sg = c.seg[c.seg_order[k]];
   const bool act = sg.status == SEG_ACTIVE;
-  v[0] = act ? sg.ntgt : 0;
+  const bool order = act && sg.tgt_mode == 1, places = order && warp_schedule(c);
+  v[0] = places ? sg.coh_n : act ? sg.ntgt : 0;
   v[1] = v[2] = 0;
-  v[3] = act && sg.tgt_mode == 1;  // summed only
+  v[3] = order && !places;  // summed only
   return 0;
 }
 __device__ int get_bound(const Ctx &c, int s, int *v)

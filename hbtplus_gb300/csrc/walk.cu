@@ -33,7 +33,7 @@ namespace {
 constexpr int kWB = 128;
 
 // Target w of this pass: segment, list position, particle, walk range.
-template <bool kRel>
+template <bool kRel, bool kWarp = false>
 __device__ __forceinline__ void load_target(const Ctx &c, int w, int total, Target &t)
 {
   if (w >= total) {
@@ -59,6 +59,10 @@ __device__ __forceinline__ void load_target(const Ctx &c, int w, int total, Targ
     pid = c.epid[epos];
     c.coh_pid[sg.off + local] = pid;
     active = true;
+  } else if (kWarp && tm == 1) {  // correction pass: the last full pass's order, still bound
+    pid = c.coh_pid[sg.off + local];
+    epos = c.epos_of_pid[pid];
+    active = (epos - sg.off) < sg.ntgt;
   } else if (tm == 1 || sg.coh_n > 0) {  // launch_bound_order, launch_list_order
     pid = c.epid2[sg.off + local];
     epos = c.epos_of_pid[pid];
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(kWB) k_walk_fp32(Ctx c, int total)
   const DevParams &P = c.P;
   const unsigned full = 0xffffffffu;
   Target t;
-  load_target<true>(c, blockIdx.x * kWB + threadIdx.x, total, t);
+  load_target<true, true>(c, blockIdx.x * kWB + threadIdx.x, total, t);
   PotAcc acc;
   const float theta2 = P.theta2;
   const float hf = P.hf, hinvf = P.hinvf, h2f = P.h2f;
