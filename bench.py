@@ -84,10 +84,10 @@ def parse():
                     help="walk_schedule option of the FP32 walk (-1: library default)")
     ap.add_argument("--small-cutoff", type=int, default=-1,
                     help="small_cutoff option: once every active subhalo's list is at most "
-                         "this long, one block per subhalo finishes the loop (-1: library "
-                         "default, 0: off)")
+                         "this long, one launch finishes the loop (-1: library default, "
+                         "0: off)")
     ap.add_argument("--small-blocks", type=int, default=-1,
-                    help="small_blocks_per_sm option (-1: library default)")
+                    help="accepted; the library's option has no effect any more")
     ap.add_argument("--scaling", default="weak", choices=["weak", "strong"],
                     help="under torchrun: weak (default) -- a global batch of N workloads, "
                          "one per rank's worth, split across the ranks by the LPT planner; "
@@ -614,10 +614,7 @@ def main():
         ub.set_option("walk_layout", args.walk_layout)
     if args.small_cutoff >= 0:
         ub.set_option("small_cutoff", args.small_cutoff)
-    if args.small_blocks >= 0:
-        ub.set_option("small_blocks_per_sm", args.small_blocks)
     small_cutoff = ub.get_option("small_cutoff")
-    small_blocks = ub.get_option("small_blocks_per_sm")
 
     stream = torch.cuda.current_stream(dev)
     ub.set_stream(stream.cuda_stream)
@@ -852,7 +849,6 @@ def main():
     line["config"]["job_particles"] = int(job["offsets"][-1])
     line["gathered_subhaloes"] = len(job_res)
     line["config"]["small_cutoff"] = small_cutoff
-    line["config"]["small_blocks_per_sm"] = small_blocks
     if rank == 0:
         print(json.dumps(line), flush=True)
     if ws > 1:
