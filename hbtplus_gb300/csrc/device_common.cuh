@@ -281,7 +281,9 @@ inline bool list_order(const Ctx &c, const PassPlan &pl)
 // particles: 937 us in pairs, 623 one by one; 1.6e5: 1014 and 967; 2.2e5: 1174 and
 // 1228; 3.4e5: 1607 and 2278; 1.1e6: 4.5 and 5.5 ms; 2.7e7: 122 and 160 ms).
 // Targets in list order are no neighbours: 780,000 of them took 810 us against 765,
-// sorted 607 against 637.
+// sorted 607 against 637.  A pass that has some of them, unsorted, takes one target per
+// lane; where they are the fewer this is the slower side (704,198 targets, 41% of them in
+// list order: first walk 2.1 ms, in pairs 1.77; from 50% on they are sorted).
 // The gradient's walk stays with one target per lane.
 constexpr int kPairMin = 152 * 4 * 5 * 64;
 inline bool pair_walk(const Ctx &c, const PassPlan &pl)

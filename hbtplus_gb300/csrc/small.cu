@@ -27,6 +27,11 @@
 // kernel and 19.8 ms in all, now 3.1 and 3.4; 400 of 20-1200: 1.93 -> 0.69 ms; one of
 // 380: 0.52 -> 0.33 ms; one of 1,920: 2.9 -> 0.75 ms.
 //
+// Registers.  Two blocks of 512 threads per SM leave 64 per thread, and the kernel
+// spills (404 bytes stored, 496 loaded in FP32 and 492 in FP64; 440 and 448 bytes of
+// stack).  Many lists need both blocks; a call of few lists has the spills on its
+// chain for nothing (another budget for those: not measured).
+//
 // Double arithmetic (frames, moments, divisions) runs at 1/64 of the FP32 rate
 // and a dependent double add takes about 150 cycles, so the steps keep it
 // off the serial chains: the moments go from the leaves up, every cell as

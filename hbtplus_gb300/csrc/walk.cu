@@ -354,10 +354,12 @@ __global__ void __launch_bounds__(kPB, 3) k_walk_fp32_pair(Ctx c, int total)
   }
 }
 
-// The walks are launched after all of the kernel before them: blocks
-// placed while its blocks still hold their SMs gather on the other SMs, and a walk
-// of few blocks never evens that out (1e5 targets after 108 blocks of 1024 threads:
-// 574 us, not 287; the unbinding of 1.1e5 particles 1.81 ms, 1.90 launched ahead).
+// The lane schedule's energy walks (these and k_walk_fp32_pair) are launched after all
+// of the kernel before them: blocks placed while its blocks still hold their SMs
+// gather on the other SMs, and a walk of few blocks never evens that out (1e5 targets
+// after 108 blocks of 1024 threads: 574 us, not 287; the unbinding of 1.1e5 particles
+// 1.81 ms, 1.90 launched ahead).  The other walks (FP64, warp schedule, gradients) are
+// launched ahead; for them the two ways have not been compared.
 template <bool kSib>
 void launch_lean(Ctx &c, int n)
 {

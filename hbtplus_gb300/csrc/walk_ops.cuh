@@ -585,8 +585,9 @@ static __device__ __noinline__ bool opens_fp64(double r2, float l2, double th2d)
 //     r^2 are fused with them.
 // All lanes of a warp call it together (lanes without a target with an empty
 // range).  Returns the potential sum (self term cancelled, before G/a).  400
-// subhaloes of up to 24,000 particles: 12.6 -> 8.6 ms a call; 1000 of up to 1900, in
-// the per-subhalo kernel: 27 -> 8.7 ms.  (Two nodes' chains interleaved: no gain.)
+// subhaloes of up to 24,000 particles: 13.0 -> 9.2 ms a call (12.6 -> 8.9 with other
+// sizes of the same law); 1000 of up to 1900, in the per-subhalo kernel: 27 -> 8.7 ms.
+// (Two nodes' chains interleaved: no gain.)
 constexpr int kFp64Queue = 8;
 
 __device__ __forceinline__ double walk_fp64(const Ctx &c, const Target &t, int *ninter)

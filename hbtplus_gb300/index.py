@@ -80,6 +80,8 @@ class _IndexTable:
         return lo.value, hi.value
 
     # -- device-resident forms (int64 CUDA tensors on the handle's device) --
+    # Work on the handle's stream: the arrays must be ready on it, and stay alive and as they
+    # are until it has passed the call (a mapped table's fill alone waits).
     def fill_device(self, keys, values, null_index: int = -1) -> None:
         self.NullIndex = int(null_index)
         _lib.check(self.lib.hbtu_index_fill(self.t, keys.data_ptr(), values.data_ptr(),

@@ -208,7 +208,8 @@ hbtu_status hbtu_set_timing(hbtu_handle *h, int32_t on);
 hbtu_status hbtu_get_stats(const hbtu_handle *h, hbtu_stats *out);
 hbtu_status hbtu_reset_stats(hbtu_handle *h);
 
-/* Tuning options of a handle (results do not depend on them):
+/* Tuning options of a handle (results do not depend on them, but for the last bits of
+ * the warp schedule's float sums):
  *   "small_cutoff"    (default 2048, at most 2048; 0: off) a call whose
  *                     subhaloes all hold at most this many particles runs in
  *                     one persistent launch, one to several warps (or blocks)
@@ -348,7 +349,10 @@ hbtu_status hbtu_index_create(hbtu_handle *h, int32_t flat, hbtu_index_table **o
 hbtu_status hbtu_index_destroy(hbtu_index_table *t);
 /* IndexTable_t::Fill(Keys, null_index) (src/hash.tpp:18-30, :59-95): the
  * pairs (keys[i], values[i]), i < n (KeyList_t::GetKey / ::GetIndex); both
- * arrays in host (location HBTU_HOST) or device memory. */
+ * arrays in host (location HBTU_HOST) or device memory.  A flat table's fill
+ * from device arrays returns before the GPU has read them, as a lookup does:
+ * they must stay as they are until the handle's stream has passed the call (a
+ * mapped table's fill waits for it). */
 hbtu_status hbtu_index_fill(hbtu_index_table *t, const int64_t *keys, const int64_t *values,
                             int64_t n, int64_t null_index, int32_t location);
 /* GetIndex for every query: out[j] = the value paired with keys[j], or the
